@@ -8,7 +8,7 @@
 // and replayed on later calls.
 #include "../../include/ifos_b200.h"
 #include "ifosb_kernels.cuh"
-#include "ifosb_tma.cuh"
+#include "ifosb_box.cuh"
 #include "ifosb_vjp.cuh"
 
 #include <cudaTypedefs.h>
@@ -130,12 +130,19 @@ struct ifosb_engine {
     int td_ck_K = 0, td_ck_nshots = 0;
     cudaError_t hook_err = cudaSuccess;
     GraphSet gtd;  // time-domain loops, one graph per batch shape and interval
-    // TMA staging (default) and its wait-timeout flag; the failure-path test knobs
+    // velocity ring: `ring` snapshots of [max_shots][3][field] beside the state's own, so
+    // that the DFT takes several steps per pass over its accumulators (attach_ring)
+    float *d_ring = nullptr;
+    int ring = 0;
+    bool ring_tried = false;
+    // TMA boxes (default; IFOSB_TMA=0: neighbours from global memory) and their
+    // wait-timeout flag; the failure-path test knobs
     int use_tma = 1;
     int *d_tma_err = nullptr;
     unsigned long long wait_ns = WAIT_LIMIT_NS;
     int stop_it = -1, stop_kernel = 0;  // stop_kernel: 1 velocity, 2 stress
-    float *d_cpg = nullptr;  // CPML rows in global memory (lane-divergent reads)
+    float *d_cpg = nullptr;  // CPML rows in global memory, their reciprocals and the z faces' per-cell rows
+    bool cpml_div = false, rho_div = false;  // CPML divisors / densities in div4's range
     // uniform relaxation times: passed as scalars instead of five model fields
     bool unif_tau = false;
     float utaus = 0.f, utaup = 0.f, uts_avg = 0.f;
@@ -158,10 +165,27 @@ static int fail(ifosb_engine *e, int code, const std::string &msg) {
                         std::string(#call) + ": " + cudaGetErrorString(_e));                         \
     } while (0)
 
+static void release_graph(GraphSet &gs);
+static void release_ring(ifosb_engine *e) {
+    if (!e->d_ring) return;
+    if (e->stream) cudaStreamSynchronize(e->stream);
+    release_graph(e->gfwd);
+    release_graph(e->gadj);
+    cudaFree(e->d_ring);
+    e->d_ring = nullptr;
+    e->dev_bytes -= (long long)sizeof(float) * e->ring * 3 * e->g.field * e->max_shots;
+    e->ring = 0;
+}
+
 template <class T>
 static int dalloc(ifosb_engine *e, T **ptr, size_t count) {
     if (count == 0) count = 1;
     cudaError_t r = cudaMalloc((void **)ptr, count * sizeof(T));
+    if (r != cudaSuccess && e->d_ring) {  // the velocity ring is only taken from memory nobody else wants
+        cudaGetLastError();
+        release_ring(e);
+        r = cudaMalloc((void **)ptr, count * sizeof(T));
+    }
     if (r != cudaSuccess) {
         *ptr = nullptr;
         cudaGetLastError();
@@ -191,6 +215,8 @@ static int dgrow(ifosb_engine *e, T **ptr, size_t *cap, size_t count) {
     return rc;
 }
 
+static bool div_range(float b) { return fabsf(b) >= DIV_B_MIN && fabsf(b) <= DIV_B_MAX; }
+
 static void fd_coeffs(int fdcoeff, float *b1, float *b2) {
     *b1 = 9.0 / 8.0; *b2 = -1.0 / 24.0;                  // Taylor (update_v_ssg.c:97)
     if (fdcoeff == 2) { *b1 = 1.1382; *b2 = -0.046414; }  // Holberg (update_v_ssg.c:98-100)
@@ -218,7 +244,7 @@ static int check_launch(ifosb_engine *e, const char *what) {
 }
 
 static int block_of(const Geo &g, int j, int i, int k) {
-    const int bx = (k - 1) / BX, by = (i - 1) / g.by, yc = (j - 1) / g.cy;
+    const int bx = (k - 1) / g.bz, by = (i - 1) / g.by, yc = (j - 1) / g.cy;
     return (yc * g.nti + by) * g.ntk + bx;
 }
 
@@ -286,9 +312,9 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
         const char *v = getenv("IFOSB_TMA");
         if (v && v[0] == '0') e->use_tma = 0;
     }
-    // tile rows: 7 (8-warp CTAs, two per SM) when the stress kernel carries memory
-    // variables, else 8; IFOSB_TILE_ROWS=7|8 overrides (tests, tuning experiments)
-    g.by = (e->use_tma && p->nmech > 0) ? 7 : 8;
+    // rows of a box (IFOSB_TILE_ROWS=7|8, IFOSB_VEL_TILE_ROWS=7|8: tests)
+    g.bz = BX;
+    g.by = TX;
     if (const char *v = getenv("IFOSB_TILE_ROWS")) {
         const int t = atoi(v);
         if (t == 7 || t == 8) g.by = t;
@@ -297,13 +323,20 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
         const int t = atoi(v);
         if (t == 7 || t == 8) e->vby = t;
     }
-    if (!e->use_tma) e->vby = g.by;
     g.ntk = (p->nz + BX - 1) / BX;
     g.nti = (p->nx + g.by - 1) / g.by;
+    {
+        // z PML rows: the near face's fw words, then the far face's, its four-cell words
+        // aligned as the cells'; a grid with a narrow interior keeps the whole row
+        const int zb = (p->fw + 3) / 4 * 4, far = p->nz - p->fw;
+        const bool whole = p->nz - 2 * p->fw < 8;
+        g.zfo = whole ? 0 : zb - far / 4 * 4;
+        g.pzw = ((whole ? p->nz : zb + far % 4 + p->fw) + 3) / 4 * 4;
+    }
     if ((long long)g.nyc * max_shots > 65535) { delete e; return IFOSB_EARG; }
-    e->sl.sx = (long long)p->ny * 2 * p->fw * p->nz;
-    e->sl.sy = (long long)2 * p->fw * p->nx * p->nz;
-    e->sl.sz = (long long)p->ny * p->nx * 2 * p->fw;
+    e->sl.sx = (long long)p->ny * 2 * p->fw * g.pz;
+    e->sl.sy = (long long)2 * p->fw * p->nx * g.pz;
+    e->sl.sz = (long long)p->ny * p->nx * g.pzw;
     e->st_shot = (long long)(NEL + 6 * p->nmech) * g.field;
     e->psi_shot = 6 * (e->sl.sx + e->sl.sy + e->sl.sz);
     e->dft_shot = (long long)max_nf * 6 * g.field;
@@ -362,7 +395,7 @@ extern "C" void ifosb_destroy(ifosb_engine *e) {
                     e->d_trig_b, e->d_voff, e->d_soff, e->d_vpts, e->d_spts, e->d_amp, e->d_tma_err, e->d_cpg,
                     e->d_mstage, e->d_green, e->d_gsig, e->d_hess, e->d_sec2, e->d_voff_t, e->d_soff_t,
                     e->d_voff_a, e->d_vpts_t, e->d_spts_t, e->d_vpts_a, e->d_amp_t, e->d_gradq, e->d_smod,
-                    e->d_td_blk, e->d_td_k};
+                    e->d_td_blk, e->d_td_k, e->d_ring};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (cudaEvent_t ev : e->events) cudaEventDestroy(ev);
@@ -432,11 +465,28 @@ extern "C" int ifosb_set_launch_mode(ifosb_engine *e, int mode) {
 
 extern "C" int ifosb_set_cpml(ifosb_engine *e, const float *coeff) {
     if (!e || !coeff) return IFOSB_EARG;
-    std::vector<float> host((size_t)18 * 2 * MAXFW, 0.f);
-    const int n2 = 2 * e->p.fw;
+    const int fw = e->p.fw, nz = e->p.nz, n2 = 2 * fw, pz = e->g.pz;
+    std::vector<float> host((size_t)CZ0 + (size_t)NCZ * pz, 0.f);
     for (int r = 0; r < 18; ++r)
         for (int h = 0; h < n2; ++h) host[(size_t)r * 2 * MAXFW + h] = coeff[(size_t)r * n2 + h];
-    CU(cudaMemcpyToSymbol(c_cpml, host.data(), host.size() * sizeof(float)));
+    auto row = [&](int r, int h) { return host[(size_t)r * 2 * MAXFW + h]; };
+    e->cpml_div = true;
+    for (int r : {K_X, KH_X, K_Y, KH_Y, K_Z, KH_Z})
+        for (int h = 0; h < n2; ++h) e->cpml_div = e->cpml_div && div_range(row(r, h));
+    for (int h = 0; h < n2; ++h) {
+        const int src[4] = {K_X, KH_X, K_Y, KH_Y}, dst[4] = {RK_X, RKH_X, RK_Y, RKH_Y};
+        for (int q = 0; q < 4; ++q) host[(size_t)dst[q] * 2 * MAXFW + h] = 1.0f / row(src[q], h);
+    }
+    for (int k = 1; k <= pz; ++k) {
+        const int h = k <= fw ? k : (k > nz - fw && k <= nz ? k - nz + n2 : 0);
+        float *c = host.data() + CZ0 + (k - 1);
+        const float kf = h ? row(K_Z, h - 1) : 1.f, kh = h ? row(KH_Z, h - 1) : 1.f;
+        const float sf = h && k <= fw ? row(K_Y, h - 1) : kf, sh = h && k <= fw ? row(KH_Y, h - 1) : kh;
+        const float v[NCZ] = {kf, 1.0f / kf, h ? row(A_Z, h - 1) : 0.f, h ? row(B_Z, h - 1) : 0.f,
+                              kh, 1.0f / kh, h ? row(AH_Z, h - 1) : 0.f, h ? row(BH_Z, h - 1) : 0.f,
+                              sf, 1.0f / sf, sh, 1.0f / sh};
+        for (int q = 0; q < NCZ; ++q) c[(size_t)q * pz] = v[q];
+    }
     if (!e->d_cpg) {
         int rc = dalloc(e, &e->d_cpg, host.size());
         if (rc) return rc;
@@ -453,10 +503,15 @@ extern "C" int ifosb_set_model(ifosb_engine *e, const float *rho, const float *p
     if (p.nmech > 0 && (!taus || !taup || !eta)) return fail(e, IFOSB_EARG, "viscoelastic model needs taus, taup, eta");
     e->ngreen = 0;  // Green's functions belong to a model
     const size_t ng = (size_t)(p.nx + 2) * (p.ny + 2) * (p.nz + 2);
-    for (size_t q = 0; q < ng; ++q)
+    float rlo = rho[0], rhi = rho[0];
+    for (size_t q = 0; q < ng; ++q) {
         if (!(rho[q] > 0.f) || !(u[q] > 0.f) || !(pi[q] > 0.f) || !std::isfinite(rho[q]) || !std::isfinite(u[q]) ||
             !std::isfinite(pi[q]))
             return fail(e, IFOSB_EARG, "model value not positive and finite at ghosted index " + std::to_string(q));
+        rlo = std::min(rlo, rho[q]);
+        rhi = std::max(rhi, rho[q]);
+    }
+    e->rho_div = rlo >= DIV_B_MIN && rhi <= DIV_B_MAX;  // and so is every average of two
     for (int l = 0; l < p.nmech; ++l)
         if (!std::isfinite(eta[l])) return fail(e, IFOSB_EARG, "eta not finite");
     if (!e->d_mstage) {  // staging for the raw model, kept for the engine's lifetime
@@ -622,7 +677,7 @@ extern "C" int ifosb_set_frequencies(ifosb_engine *e, int nf, const float *finv,
 // ---------------------------------------------------------------------------
 // the time loop
 
-static_assert(TZ == BX, "TMA tiles and plain blocks share one block geometry along z");
+static_assert(TZ == BX && TX == BY, "boxes and the gradient's blocks share the engine's geometry");
 
 // Everything one forward or adjoint call launches with.
 // The time-domain checkpoints an armed forward writes after its steps: the
@@ -639,12 +694,22 @@ struct Loop {
     Geo lgv;  // launch geometry of the velocity kernel
     VelArgs va;
     StrArgs sa;
-    VelTma vt;
-    StrTma stt;
+    VelBox vt;
+    StrBox stt;
+    DftArgs da;
+    // velocity slots 0 (the state's own) .. ring-1, the DFT's accumulators and tables, and
+    // the slot the loop starts from (so that it ends in slot 0)
+    int ring, first;
+    float *slot[MAXRING];
+    long long slot_shot[MAXRING];
+    CUtensorMap vmap[MAXRING], smap[MAXRING];
+    float *dft;
+    const double *trig;
     int nshots = 0;
     bool back = false;
     bool tma = false;
     bool p2 = false;  // power-of-two spacings (stress kernel multiplies by 1/DX etc.)
+    int yb = 0;       // quad kernels: planes of a block (lg.cy / yb of them per thread)
     size_t vel_smem = 0, str_smem = 0;
     TdHook td;
 };
@@ -661,33 +726,42 @@ static const ifosb_engine::Shape *shape_for(const ifosb_engine *e, int nshots) {
     return &hi->second;
 }
 
-// y planes per CTA. Untuned, with no other batch size tuned either: enough chunks
-// for about four CTAs per SM over the whole batch, 8 to 16 planes each (the
-// autotuner picked 3 to 32 on 128^3 to 384x256x384 grids; chunks of 64 planes ran
-// a 10-shot 384x256x384 batch 60 % slower than its tuned shape).
-static Geo launch_geo(const ifosb_engine *e, int nshots, bool vel) {
+// The box kernels' geometry: y planes per CTA, one box unless a launch shape says more.
+static Geo box_geo(const ifosb_engine *e, int nshots, bool vel) {
     Geo g = e->g;
     if (vel) {
         g.by = e->vby;
         g.nti = (g.nx + g.by - 1) / g.by;
     }
-    int cy;
-    if (const ifosb_engine::Shape *t = shape_for(e, nshots)) {
-        cy = vel ? t->cyv : t->cys;
-    } else {
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaGetLastError();
-        const long long per_set = (long long)g.ntk * g.nti * nshots;
-        const long long chunks = std::max<long long>(1, (4LL * sms + per_set - 1) / per_set);
-        cy = (int)((g.ny + chunks - 1) / chunks);
-        cy = std::min(std::max(cy, DEFAULT_CY), 16);
-    }
-    cy = std::min(cy, g.ny);
+    const int yb = vel ? VYB : str_yb(g.nmech);
+    const ifosb_engine::Shape *t = shape_for(e, nshots);
+    int cy = std::min(t ? (vel ? t->cyv : t->cys) : yb, g.ny);
     while (cy < g.ny && (long long)((g.ny + cy - 1) / cy) * nshots > 65535) ++cy;  // grid.z limit
     g.cy = cy;
     g.nyc = (g.ny + cy - 1) / cy;
     return g;
+}
+
+// The quad kernels' geometry: blocks of at most 8 quads (z) x 8 rows x 4 planes, the
+// extents evened out over each axis so that the last block of a row is not nearly empty.
+static Geo quad_geo(const ifosb_engine *e, int nshots, int &yb) {
+    Geo g = e->g;
+    auto even = [](int n, int most) { const int b = (n + most - 1) / most; return (n + b - 1) / b; };
+    const int nq = (g.nz + 3) / 4, bq = even(nq, QZ);
+    g.bz = 4 * bq;
+    g.ntk = (nq + bq - 1) / bq;
+    g.by = even(g.nx, QX);
+    g.nti = (g.nx + g.by - 1) / g.by;
+    yb = g.cy = even(g.ny, QTHR / QZ / QX);
+    while ((long long)((g.ny + g.cy - 1) / g.cy) * nshots > 65535) g.cy += yb;  // grid.z limit
+    g.nyc = (g.ny + g.cy - 1) / g.cy;
+    return g;
+}
+
+// An exact reciprocal exists for a power-of-two spacing: x/h == x*(1/h) bit for bit.
+static bool pow2(float h) {
+    int ex = 0;
+    return h > 0.f && std::isfinite(h) && std::frexp(h, &ex) == 0.5f;
 }
 
 static void fill_common(ifosb_engine *e, Loop &L) {
@@ -719,6 +793,13 @@ static void fill_common(ifosb_engine *e, Loop &L) {
     }
     va.err_step = e->d_err;
     va.cpg = sa.cpg = e->d_cpg;
+    va.rho = e->d_rho_w;
+    va.fast_div = e->cpml_div && e->rho_div;
+    sa.fast_div = e->cpml_div && div_range(p.dx) && div_range(p.dy) && div_range(p.dz);
+    sa.unif_tau = e->unif_tau;
+    sa.utaus = e->utaus; sa.utaup = e->utaup; sa.uts_avg = e->uts_avg;
+    sa.idx = 1.0f / p.dx; sa.idy = 1.0f / p.dy; sa.idz = 1.0f / p.dz;
+    L.p2 = pow2(p.dx) && pow2(p.dy) && pow2(p.dz);
     va.probe_j = p.ny / 2; va.probe_i = p.nx / 2; va.probe_k = p.nz / 2;  // ifos3d.c:761
     sa.dt = p.dt;
     sa.dthalbe = p.dt / 2.0;
@@ -739,8 +820,9 @@ static void fill_common(ifosb_engine *e, Loop &L) {
     sa.sec_tr = e->ns;
     sa.sec_comp = (long long)e->ntr * e->ns;
     sa.sec_shot = 3 * sa.sec_comp;
-    sa.nf = e->nf;
-    sa.dft_shot = e->dft_shot;
+    va.vin = va.vout = e->d_state;
+    sa.v = e->d_state;
+    va.vin_shot = va.vout_shot = sa.v_shot = e->st_shot;
     sa.smod = e->smod_on ? e->d_smod : nullptr;
 }
 
@@ -773,153 +855,243 @@ static void smem_set(const void *f, size_t bytes) {
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 template <int M>
-static void smem_attrs(int vby, int sby, size_t vel, size_t str) {
-    if (vby == 7) {
-        smem_set((const void *)t7::k_velocity_tma<true>, vel);
-        smem_set((const void *)t7::k_velocity_tma<false>, vel);
-    } else {
-        smem_set((const void *)t8::k_velocity_tma<true>, vel);
-        smem_set((const void *)t8::k_velocity_tma<false>, vel);
-    }
-    if (sby == 7) {
-        smem_set((const void *)t7::k_stress_tma<M, true>, str);
-        smem_set((const void *)t7::k_stress_tma<M, false>, str);
-    } else {
-        smem_set((const void *)t8::k_stress_tma<M, true>, str);
-        smem_set((const void *)t8::k_stress_tma<M, false>, str);
-    }
+static void smem_attrs(size_t vel, size_t str) {
+    smem_set((const void *)k_velocity_box<true>, vel);
+    smem_set((const void *)k_velocity_box<false>, vel);
+    smem_set((const void *)k_stress_box<M, true>, str);
+    smem_set((const void *)k_stress_box<M, false>, str);
 }
 
-// An exact reciprocal exists for a power-of-two spacing: x/h == x*(1/h) bit for bit.
-static bool pow2(float h) {
-    int ex = 0;
-    return h > 0.f && std::isfinite(h) && std::frexp(h, &ex) == 0.5f;
-}
-
-// Tensor maps over the state [shot][slot][y][x][z], the model [slot][y][x][z] and the
-// DFT accumulators [shot][6 nf][y][x][z]; false if TMA staging cannot be used.
-static bool setup_tma(ifosb_engine *e, Loop &L, float *dft) {
+// The box kernels' tensor maps over the state [shot][slot][y][x][z], the model
+// [slot][y][x][z] and rho, and their launch constants; false if they cannot be used.
+static bool setup_tma(ifosb_engine *e, Loop &L) {
     const Geo &g = e->g;
     const ifosb_params &p = e->p;
     const int nslot = NEL + 6 * p.nmech;
     const int nsr = 6 + 6 * p.nmech;
     const int nm = (p.nmech == 0 || e->unif_tau) ? 5 : 10;
-    const int ndf = (dft && e->nf > 0) ? 6 * e->nf : 0;
-    const size_t vs = L.lgv.by == 7 ? t7::vel_tma_smem() : t8::vel_tma_smem();
-    const size_t ss = L.lg.by == 7 ? t7::str_tma_smem(nsr, nm, ndf) : t8::str_tma_smem(nsr, nm, ndf);
-    const cuuint32_t TXV = (cuuint32_t)L.lgv.by, RXV = TXV + 2 * HX;  // velocity tile rows, ring rows
-    const cuuint32_t TX = (cuuint32_t)L.lg.by, RX = TX + 2 * HX;      // stress tile rows, ring rows
-    if (vs > 227 * 1024 || ss > 227 * 1024) return false;
+    const cuuint32_t yb = (cuuint32_t)str_yb(p.nmech);
+    const size_t vs = 4 * (size_t)VelSm<VYB>::END;
+    const size_t ss = yb == 4 ? str_box_bytes<4>(nsr, nm) : str_box_bytes<2>(nsr, nm);
+    if (vs > 226 * 1024 || ss > 226 * 1024) return false;
     const cuuint64_t sdims[5] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(p.ny + 5), (cuuint64_t)nslot,
-                                 (cuuint64_t)e->max_shots};
+                                 (cuuint64_t)L.nshots};
     const cuuint64_t sstr[4] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)g.field * 4,
                                 (cuuint64_t)e->st_shot * 4};
     const cuuint64_t mdims[4] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(p.ny + 5), (cuuint64_t)NMODEL};
     const cuuint64_t mstr[3] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)g.field * 4};
-    const cuuint32_t bhalov[5] = {(cuuint32_t)RZ, RXV, 1, 3, 1}, bpt[5] = {(cuuint32_t)TZ, TXV, 1, 3, 1};
-    const cuuint64_t rdims[3] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(p.ny + 5)};
-    const cuuint64_t rstr[2] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.plane * 4};
-    const cuuint32_t brh[3] = {(cuuint32_t)RZ, RXV, 1}, brp[3] = {(cuuint32_t)TZ, TXV, 1};
-    const cuuint32_t bhalo[5] = {(cuuint32_t)RZ, RX, 1, 3, 1}, bsr[5] = {(cuuint32_t)TZ, TX, 1, (cuuint32_t)nsr, 1};
-    const cuuint32_t bms[4] = {(cuuint32_t)TZ, TX, 1, (cuuint32_t)nm};
-    L.vt = VelTma{};
-    L.stt = StrTma{};
-    if (!encode(&L.vt.m_halo, e->d_state, 5, sdims, sstr, bhalov) ||
-        !encode(&L.vt.m_pt, e->d_state, 5, sdims, sstr, bpt) ||
-        !encode(&L.vt.m_rho_halo, e->d_rho_w, 3, rdims, rstr, brh) ||
-        !encode(&L.vt.m_rho_pt, e->d_rho_w, 3, rdims, rstr, brp) ||
-        !encode(&L.stt.m_halo, e->d_state, 5, sdims, sstr, bhalo) ||
-        !encode(&L.stt.m_sr, e->d_state, 5, sdims, sstr, bsr) || !encode(&L.stt.m_mod, e->d_model, 4, mdims, mstr, bms))
+    auto state = [&](CUtensorMap *m, cuuint32_t z, cuuint32_t x, cuuint32_t y, cuuint32_t slots) {
+        const cuuint32_t box[5] = {z, x, y, slots, 1};
+        return encode(m, e->d_state, 5, sdims, sstr, box);
+    };
+    VelBox &v = L.vt;
+    StrBox &t = L.stt;
+    const cuuint32_t brho[3] = {WR, TX + 1, VYB + 1}, bmod[4] = {TZ, TX, yb, (cuuint32_t)nm};
+    if (!state(&v.xx, TZ, XH, VYB, 1) || !state(&v.zz, WZ, TX, VYB, 1) || !state(&v.xz, WZ, XH, VYB, 1) ||
+        !state(&v.yy, TZ, TX, VYB + 3, 1) || !state(&v.xy, TZ, XH, VYB + 3, 1) || !state(&v.yz, WZ, TX, VYB + 3, 1) ||
+        !encode(&v.rho, e->d_rho_w, 3, mdims, mstr, brho) || !state(&t.sr, TZ, TX, yb, (cuuint32_t)nsr) || !encode(&t.mod, e->d_model, 4, mdims, mstr, bmod))
         return false;
-    if (ndf) {
-        const cuuint64_t ddims[5] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(p.ny + 5),
-                                     (cuuint64_t)(6 * e->max_nf), (cuuint64_t)e->max_shots};
-        const cuuint64_t dstr[4] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)g.field * 4,
-                                    (cuuint64_t)e->dft_shot * 4};
-        const cuuint32_t bd[5] = {(cuuint32_t)TZ, TX, 1, (cuuint32_t)ndf, 1};
-        if (!encode(&L.stt.m_dft, dft, 5, ddims, dstr, bd)) return false;
+    v.tma_err = t.tma_err = e->d_tma_err;
+    v.w = WaitCtl{e->wait_ns, e->stop_kernel == 1 ? e->stop_it : -1};
+    t.w = WaitCtl{e->wait_ns, e->stop_kernel == 2 ? e->stop_it : -1};
+    if (const ifosb_engine::Shape *sh = shape_for(e, L.nshots)) {
+        v.ahead = sh->l2v;
+        t.ahead = sh->l2s;
     }
-    L.vt.a = L.va;
-    L.stt.a = L.sa;
-    L.vt.tma_err = L.stt.tma_err = e->d_tma_err;
-    L.vt.w = WaitCtl{e->wait_ns, e->stop_kernel == 1 ? e->stop_it : -1};
-    L.stt.w = WaitCtl{e->wait_ns, e->stop_kernel == 2 ? e->stop_it : -1};
-    {
-        const ifosb_engine::Shape *t = shape_for(e, L.nshots);
-        L.vt.l2ahead = t ? t->l2v : L2AHEAD_VEL_DEFAULT;
-        L.stt.l2ahead = t ? t->l2s : L2AHEAD_STR_DEFAULT;
-    }
-    L.stt.nsr = nsr;
-    L.stt.nm = nm;
-    L.stt.ndf = ndf;
-    L.stt.utaus = e->utaus;
-    L.stt.utaup = e->utaup;
-    L.stt.uts_avg = e->uts_avg;
-    L.p2 = pow2(p.dx) && pow2(p.dy) && pow2(p.dz);
-    L.stt.idx = 1.0f / p.dx;
-    L.stt.idy = 1.0f / p.dy;
-    L.stt.idz = 1.0f / p.dz;
+    t.nsr = nsr;
+    t.nm = nm;
     L.vel_smem = vs;
     L.str_smem = ss;
     switch (p.nmech) {
-    case 0: smem_attrs<0>(L.lgv.by, L.lg.by, vs, ss); break;
-    case 1: smem_attrs<1>(L.lgv.by, L.lg.by, vs, ss); break;
-    case 2: smem_attrs<2>(L.lgv.by, L.lg.by, vs, ss); break;
-    case 3: smem_attrs<3>(L.lgv.by, L.lg.by, vs, ss); break;
-    default: smem_attrs<4>(L.lgv.by, L.lg.by, vs, ss); break;
+    case 0: smem_attrs<0>(vs, ss); break;
+    case 1: smem_attrs<1>(vs, ss); break;
+    case 2: smem_attrs<2>(vs, ss); break;
+    case 3: smem_attrs<3>(vs, ss); break;
+    default: smem_attrs<4>(vs, ss); break;
     }
     return cudaGetLastError() == cudaSuccess;
 }
 
-template <int M>
-static void launch_str_m(const Loop &L, dim3 grd, cudaStream_t st, int nt, int do_dft, int sample) {
-    const int by = L.lg.by;
+// Picks the kernels and the launch geometry of a time loop over the engine's state.
+static void plan_loop(ifosb_engine *e, Loop &L, int nshots, bool back) {
+    std::memset(static_cast<void *>(&L), 0, sizeof(L));  // the graph cache compares Loops bytewise, padding included
+    L.nshots = nshots;
+    L.back = back;
+    L.tma = e->use_tma && setup_tma(e, L);
     if (L.tma) {
-        const dim3 blk(TZ, by + 1);
-        if (by == 7) {
-            if (L.p2) t7::k_stress_tma<M, true><<<grd, blk, L.str_smem, st>>>(L.stt, nt, do_dft, sample);
-            else t7::k_stress_tma<M, false><<<grd, blk, L.str_smem, st>>>(L.stt, nt, do_dft, sample);
-        } else {
-            if (L.p2) t8::k_stress_tma<M, true><<<grd, blk, L.str_smem, st>>>(L.stt, nt, do_dft, sample);
-            else t8::k_stress_tma<M, false><<<grd, blk, L.str_smem, st>>>(L.stt, nt, do_dft, sample);
-        }
+        L.lg = box_geo(e, nshots, false);
+        L.lgv = box_geo(e, nshots, true);
     } else {
-        k_stress<M><<<grd, dim3(BX, by), 0, st>>>(L.sa, nt, do_dft, sample);
+        L.lg = L.lgv = quad_geo(e, nshots, L.yb);
     }
 }
 
-static void launch_str(int nmech, const Loop &L, dim3 grd, cudaStream_t st, int nt, int do_dft, int sample) {
+// DFT steps: nt % ntast == 0 (ifos3d.c:788).
+static bool dft_step(const ifosb_engine *e, int nt) { return e->nf > 0 && nt % e->ntast == 0; }
+
+// The velocity ring of a loop that accumulates DFT fields. Called last before the loop,
+// when everything else it needs is allocated: the ring takes at most half of the device
+// memory that is free then, in snapshots of the whole batch, up to MAXRING with the
+// state's own (a 384x256x384, L = 3, nf = 4 shot: 2.70 ms per step with 8), and is
+// given back when any later allocation of the engine fails. The time-domain checkpoints
+// of an armed forward read the state's own velocities after every step: no ring.
+static int attach_ring(ifosb_engine *e, Loop &L) {
+    L.ring = 1;
+    L.slot[0] = e->d_state;
+    L.slot_shot[0] = e->st_shot;
+    const long long F = e->g.field;
+    if (L.dft && e->nf > 0 && L.td.K == 0) {
+        const int want = std::min(MAXRING, e->p.nt / e->ntast) - 1;  // no more snapshots than DFT steps
+        const size_t one = sizeof(float) * 3 * (size_t)F * e->max_shots;
+        if (!e->d_ring && want > 0 && !e->ring_tried) {
+            size_t free_b = 0, total_b = 0;
+            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+            int n = (int)std::min<size_t>(want, free_b / 2 / one);
+            if (n > 0 && cudaMalloc((void **)&e->d_ring, n * one) != cudaSuccess) n = 0;
+            cudaGetLastError();
+            e->ring_tried = true;  // one look per engine: a batch keeps its launch graphs
+            if (n > 0) {
+                e->ring = n;
+                e->dev_bytes += (long long)(n * one);
+                CU(cudaMemsetAsync(e->d_ring, 0, n * one, e->stream));  // halos stay zero
+            } else {
+                e->d_ring = nullptr;
+            }
+        }
+        L.ring = 1 + std::max(0, std::min(want, e->ring));
+        for (int r = 1; r < L.ring; ++r) {
+            L.slot[r] = e->d_ring + (size_t)(r - 1) * 3 * F * e->max_shots;
+            L.slot_shot[r] = 3 * F;
+        }
+    }
+    // a step after a DFT step whose velocities are still wanted goes to the next slot
+    int moves = 0, held = 0;
+    for (int nt = 1; nt < e->p.nt; ++nt)
+        if (dft_step(e, nt) && L.ring > 1) {
+            if (++held == L.ring) held = 0;
+            else ++moves;
+        }
+    L.first = (L.ring - moves % L.ring) % L.ring;
+    if (L.first) CU(cudaMemsetAsync(L.slot[L.first], 0, sizeof(float) * 3 * (size_t)F * L.nshots, e->stream));
+    if (L.tma) {
+        const Geo &g = e->g;
+        const cuuint32_t yb = (cuuint32_t)str_yb(e->p.nmech);
+        for (int r = 0; r < L.ring; ++r) {
+            const cuuint64_t dims[5] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(e->p.ny + 5), 3, (cuuint64_t)L.nshots};
+            const cuuint64_t str[4] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)F * 4, (cuuint64_t)L.slot_shot[r] * 4};
+            const cuuint32_t bv[5] = {TZ, TX, VYB, 3, 1}, bs[5] = {WZ, XH, yb + 3, 1, 1};
+            if (!encode(&L.vmap[r], L.slot[r], 5, dims, str, bv) || !encode(&L.smap[r], L.slot[r], 5, dims, str, bs))
+                return fail(e, IFOSB_ECUDA, "tensor map of the velocities");
+        }
+    }
+    return IFOSB_OK;
+}
+
+// The kernel arguments of a planned loop, once va and sa are complete.
+static int finish_plan(ifosb_engine *e, Loop &L) {
+    L.vt.a = L.va;
+    L.stt.a = L.sa;
+    L.da.g = e->g;
+    L.da.dft = L.dft;
+    L.da.dft_shot = e->dft_shot;
+    L.da.nf = e->nf;
+    return attach_ring(e, L);
+}
+
+// The velocities of a step: read from slot `in`, written to slot `out`.
+static void set_slots(Loop &L, int in, int out) {
+    L.va.vin = L.vt.a.vin = L.slot[in];
+    L.va.vin_shot = L.vt.a.vin_shot = L.slot_shot[in];
+    L.va.vout = L.vt.a.vout = L.slot[out];
+    L.va.vout_shot = L.vt.a.vout_shot = L.slot_shot[out];
+    L.sa.v = L.stt.a.v = L.slot[out];
+    L.sa.v_shot = L.stt.a.v_shot = L.slot_shot[out];
+    L.vt.v = L.vmap[in];
+    L.stt.v = L.smap[out];
+}
+
+template <int P>
+static void launch_dft_p(const DftArgs &a, dim3 grd, cudaStream_t st) {
+    k_dft<P><<<grd, 128, 0, st>>>(a);
+}
+
+// Which slots hold velocities the DFT has not taken yet; a pass when the ring is full
+// or the loop ends.
+struct DftRing {
+    int cur = 0, n = 0, held[MAXRING] = {}, step[MAXRING] = {};
+    bool last_held = false;
+    void before(Loop &L) {
+        const int out = last_held ? (cur + 1) % L.ring : cur;
+        set_slots(L, cur, out);
+        cur = out;
+    }
+    void after(ifosb_engine *e, Loop &L, int nt) {
+        last_held = false;
+        if (L.dft && dft_step(e, nt)) {
+            held[n] = cur;
+            step[n++] = nt;
+            last_held = true;
+        }
+        if (n == 0 || (n < L.ring && nt < e->p.nt)) return;
+        for (int p = 0; p < n; ++p) {
+            L.da.v[p] = L.slot[held[p]];
+            L.da.v_shot[p] = L.slot_shot[held[p]];
+            L.da.trig[p] = L.trig + (size_t)(step[p] - 1) * e->nf * 2;
+        }
+        const long long quads = (long long)((e->g.nz + 3) / 4) * e->g.nx * e->g.ny;
+        const dim3 grd((unsigned)((quads + 127) / 128), 3, L.nshots);
+        switch (n) {
+        case 1: launch_dft_p<1>(L.da, grd, e->stream); break;
+        case 2: launch_dft_p<2>(L.da, grd, e->stream); break;
+        case 3: launch_dft_p<3>(L.da, grd, e->stream); break;
+        case 4: launch_dft_p<4>(L.da, grd, e->stream); break;
+        case 5: launch_dft_p<5>(L.da, grd, e->stream); break;
+        case 6: launch_dft_p<6>(L.da, grd, e->stream); break;
+        case 7: launch_dft_p<7>(L.da, grd, e->stream); break;
+        default: launch_dft_p<8>(L.da, grd, e->stream); break;
+        }
+        n = 0;
+        last_held = false;
+    }
+};
+
+template <int M>
+static void launch_str_m(const Loop &L, dim3 grd, cudaStream_t st, int nt, int sample) {
+    if (L.tma) {
+        const int thr = 64 * str_yb(M);
+        if (L.p2) k_stress_box<M, true><<<grd, thr, L.str_smem, st>>>(L.stt, nt, sample);
+        else k_stress_box<M, false><<<grd, thr, L.str_smem, st>>>(L.stt, nt, sample);
+    } else {
+        const int thr = L.lg.bz / 4 * L.lg.by * L.yb;
+        if (L.p2) k_stress<M, true><<<grd, thr, 0, st>>>(L.sa, nt, sample, L.yb);
+        else k_stress<M, false><<<grd, thr, 0, st>>>(L.sa, nt, sample, L.yb);
+    }
+}
+
+static void launch_str(int nmech, const Loop &L, dim3 grd, cudaStream_t st, int nt, int sample) {
     switch (nmech) {
-    case 0: launch_str_m<0>(L, grd, st, nt, do_dft, sample); break;
-    case 1: launch_str_m<1>(L, grd, st, nt, do_dft, sample); break;
-    case 2: launch_str_m<2>(L, grd, st, nt, do_dft, sample); break;
-    case 3: launch_str_m<3>(L, grd, st, nt, do_dft, sample); break;
-    default: launch_str_m<4>(L, grd, st, nt, do_dft, sample); break;
+    case 0: launch_str_m<0>(L, grd, st, nt, sample); break;
+    case 1: launch_str_m<1>(L, grd, st, nt, sample); break;
+    case 2: launch_str_m<2>(L, grd, st, nt, sample); break;
+    case 3: launch_str_m<3>(L, grd, st, nt, sample); break;
+    default: launch_str_m<4>(L, grd, st, nt, sample); break;
     }
 }
 
 static void launch_vel(const Loop &L, dim3 grd, cudaStream_t st, int nt) {
-    const int by = L.lgv.by;
     if (L.tma) {
-        const dim3 blk(TZ, by + 1);
-        if (by == 7) {
-            if (L.back) t7::k_velocity_tma<true><<<grd, blk, L.vel_smem, st>>>(L.vt, nt);
-            else t7::k_velocity_tma<false><<<grd, blk, L.vel_smem, st>>>(L.vt, nt);
-        } else {
-            if (L.back) t8::k_velocity_tma<true><<<grd, blk, L.vel_smem, st>>>(L.vt, nt);
-            else t8::k_velocity_tma<false><<<grd, blk, L.vel_smem, st>>>(L.vt, nt);
-        }
+        if (L.back) k_velocity_box<true><<<grd, 64 * VYB, L.vel_smem, st>>>(L.vt, nt);
+        else k_velocity_box<false><<<grd, 64 * VYB, L.vel_smem, st>>>(L.vt, nt);
     } else {
-        const dim3 blk(BX, by);
-        if (L.back) k_velocity<true><<<grd, blk, 0, st>>>(L.va, nt);
-        else k_velocity<false><<<grd, blk, 0, st>>>(L.va, nt);
+        const int thr = L.lgv.bz / 4 * L.lgv.by * L.yb;
+        if (L.back) k_velocity<true><<<grd, thr, 0, st>>>(L.va, nt, L.yb);
+        else k_velocity<false><<<grd, thr, 0, st>>>(L.va, nt, L.yb);
     }
 }
 
-// Per-step launch parameters: DFT on steps nt % ntast == 0 (ifos3d.c:788), seismogram
-// sample index when nt == lsamp (ifos3d.c:799-804, forward only).
-static void step_flags(const ifosb_engine *e, bool back, int nt, int &lsamp, int &nlsamp, int &do_dft, int &sample) {
-    do_dft = (e->nf > 0 && nt % e->ntast == 0) ? 1 : 0;
+// Per-step launch parameters: seismogram sample index when nt == lsamp (ifos3d.c:799-804,
+// forward only).
+static void step_flags(const ifosb_engine *e, bool back, int nt, int &lsamp, int &nlsamp, int &sample) {
     sample = -1;
     if (!back && nt == lsamp) {
         sample = nlsamp++;
@@ -980,22 +1152,31 @@ static void td_hook(ifosb_engine *e, const Loop &L, int nt) {
     if (nt == e->p.nt) hook_copy(e, t.uf_end, t.uf, t.us);
 }
 
-// Enqueue the NT steps (two kernels per step) on the engine stream.
-static void enqueue_loop(ifosb_engine *e, const Loop &L) {
+// Enqueue the NT steps (two kernels per step, and the DFT passes) on the engine stream.
+static void enqueue_loop(ifosb_engine *e, const Loop &plan) {
+    Loop L = plan;
+    DftRing ring;
+    ring.cur = L.first;
     const ifosb_params &p = e->p;
     const dim3 grd(L.lg.ntk, L.lg.nti, L.lg.nyc * L.nshots), grdv(L.lgv.ntk, L.lgv.nti, L.lgv.nyc * L.nshots);
     int lsamp = p.ndtshift + 1, nlsamp = 0;
     for (int nt = 1; nt <= p.nt; ++nt) {
+        ring.before(L);
         launch_vel(L, grdv, e->stream, nt);
-        int do_dft, sample;
-        step_flags(e, L.back, nt, lsamp, nlsamp, do_dft, sample);
-        launch_str(p.nmech, L, grd, e->stream, nt, do_dft, sample);
+        int sample;
+        step_flags(e, L.back, nt, lsamp, nlsamp, sample);
+        launch_str(p.nmech, L, grd, e->stream, nt, sample);
+        ring.after(e, L, nt);
         if (L.td.K) td_hook(e, L, nt);
     }
 }
 
-// Kernel-by-kernel launches with an event pair around each kernel (kernel timing).
-static int run_loop_profiled(ifosb_engine *e, const Loop &L) {
+// Kernel-by-kernel launches with an event pair around each kernel (kernel timing; the
+// stress time includes the step's DFT pass).
+static int run_loop_profiled(ifosb_engine *e, const Loop &plan) {
+    Loop L = plan;
+    DftRing ring;
+    ring.cur = L.first;
     const ifosb_params &p = e->p;
     const int nsteps = e->nt_limit > 0 ? std::min(e->nt_limit, p.nt) : p.nt;  // the autotuner times a few steps
     const size_t need = (size_t)3 * nsteps;
@@ -1009,11 +1190,13 @@ static int run_loop_profiled(ifosb_engine *e, const Loop &L) {
     for (int nt = 1; nt <= nsteps; ++nt) {
         cudaEvent_t *ev = &e->events[(size_t)3 * (nt - 1)];
         CU(cudaEventRecord(ev[0], e->stream));
+        ring.before(L);
         launch_vel(L, grdv, e->stream, nt);
         CU(cudaEventRecord(ev[1], e->stream));
-        int do_dft, sample;
-        step_flags(e, L.back, nt, lsamp, nlsamp, do_dft, sample);
-        launch_str(p.nmech, L, grd, e->stream, nt, do_dft, sample);
+        int sample;
+        step_flags(e, L.back, nt, lsamp, nlsamp, sample);
+        launch_str(p.nmech, L, grd, e->stream, nt, sample);
+        ring.after(e, L, nt);
         CU(cudaEventRecord(ev[2], e->stream));
         if (L.td.K) td_hook(e, L, nt);
     }
@@ -1073,7 +1256,8 @@ static int replay_graph(ifosb_engine *e, GraphSet &gs, const std::vector<unsigne
 
 static int run_loop(ifosb_engine *e, const Loop &L) {
     GraphSet &gs = L.back ? e->gadj : e->gfwd;
-    e->launches = 2LL * e->p.nt;
+    const int dft_steps = L.dft && e->nf > 0 ? e->p.nt / e->ntast : 0;
+    e->launches = 2LL * e->p.nt + (dft_steps + L.ring - 1) / L.ring;
     if (e->profile) return run_loop_profiled(e, L);
     if (e->launch_mode == 1) {
         enqueue_loop(e, L);
@@ -1149,11 +1333,7 @@ extern "C" int ifosb_forward(ifosb_engine *e, int nshots, const ifosb_shot *shot
         for (int t = 0; t < e->ntr; ++t) sp.push_back({s, e->rec[3 * t + 1], e->rec[3 * t], e->rec[3 * t + 2], PT_RECEIVER, t});
     }
     Loop L;
-    std::memset(static_cast<void *>(&L), 0, sizeof(L));  // the graph cache compares Loops bytewise, padding included
-    L.nshots = nshots;
-    L.back = false;
-    L.lg = launch_geo(e, nshots, false);
-    L.lgv = launch_geo(e, nshots, true);
+    plan_loop(e, L, nshots, false);
     int rc;
     if ((rc = upload_points(e, L.lgv, nshots, vp, &e->d_voff, &e->cap_voff, &e->d_vpts, &e->cap_vpts)) ||
         (rc = upload_points(e, L.lg, nshots, sp, &e->d_soff, &e->cap_soff, &e->d_spts, &e->cap_spts)) ||
@@ -1176,9 +1356,8 @@ extern "C" int ifosb_forward(ifosb_engine *e, int nshots, const ifosb_shot *shot
     sa.pts = e->d_spts;
     sa.amp = e->d_amp;
     sa.amp_row = p.nt;
-    sa.dft = e->d_dftf;
-    sa.trig = e->d_trig_f;
-    L.tma = e->use_tma && setup_tma(e, L, e->d_dftf);
+    L.dft = e->d_dftf;
+    L.trig = e->d_trig_f;
     e->fwd_ok = e->res_ok = e->adj_ok = e->hess_fwd = false;
     e->td_ck_ok = false;
     TdLayout tl;
@@ -1189,6 +1368,7 @@ extern "C" int ifosb_forward(ifosb_engine *e, int nshots, const ifosb_shot *shot
         L.td = TdHook{uf, uf_end, uf_end + tl.us, tl.ck, tl.ss, tl.ps, tl.us, tl.ssz, tl.psz, tl.K, tl.nseg};
         CU(cudaMemsetAsync(uf, 0, tl.us * sizeof(float), e->stream));
     }
+    if ((rc = finish_plan(e, L))) return rc;
     e->hook_err = cudaSuccess;
     if ((rc = run_loop(e, L))) return rc;
     if (e->hook_err != cudaSuccess)
@@ -1254,11 +1434,7 @@ extern "C" int ifosb_adjoint(ifosb_engine *e, const float *diff) {
     for (int s = 0; s < nshots; ++s)
         for (int t = 0; t < ntr; ++t) vp.push_back({s, e->rec[3 * t + 1], e->rec[3 * t], e->rec[3 * t + 2], PT_ADJOINT, s * 3 * ntr + t});
     Loop L;
-    std::memset(static_cast<void *>(&L), 0, sizeof(L));  // the graph cache compares Loops bytewise, padding included
-    L.nshots = nshots;
-    L.back = true;
-    L.lg = launch_geo(e, nshots, false);
-    L.lgv = launch_geo(e, nshots, true);
+    plan_loop(e, L, nshots, true);
     int rc;
     if ((rc = upload_points(e, L.lgv, nshots, vp, &e->d_voff, &e->cap_voff, &e->d_vpts, &e->cap_vpts))) return rc;
     if ((rc = reset_state(e, nshots, e->d_dftb))) return rc;
@@ -1272,10 +1448,9 @@ extern "C" int ifosb_adjoint(ifosb_engine *e, const float *diff) {
     va.val_comp = (long long)ntr * ns;
     sa.pt_off = nullptr;
     sa.pts = nullptr;
-    sa.dft = e->d_dftb;
-    sa.trig = e->d_trig_b;
-    L.tma = e->use_tma && setup_tma(e, L, e->d_dftb);
-    if ((rc = run_loop(e, L))) return rc;
+    L.dft = e->d_dftb;
+    L.trig = e->d_trig_b;
+    if ((rc = finish_plan(e, L)) || (rc = run_loop(e, L))) return rc;
     if ((rc = check_unstable(e, nshots))) return rc;
     e->adj_ok = true;
     return check_launch(e, "adjoint");
@@ -1349,7 +1524,7 @@ extern "C" int ifosb_gradient(ifosb_engine *e) {
 static void td_step(ifosb_engine *e, const Loop &L, int nt) {
     const dim3 grd(L.lg.ntk, L.lg.nti, L.lg.nyc * L.nshots), grdv(L.lgv.ntk, L.lgv.nti, L.lgv.nyc * L.nshots);
     launch_vel(L, grdv, e->stream, nt);
-    launch_str(e->p.nmech, L, grd, e->stream, nt, 0, -1);
+    launch_str(e->p.nmech, L, grd, e->stream, nt, -1);
 }
 
 extern "C" int ifosb_set_td_checkpoints(ifosb_engine *e, int interval) {
@@ -1384,11 +1559,13 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
     int rc = IFOSB_OK;
     auto run = [&]() -> int {
         // the recomputation loop: the last forward's sources on its own state
+        std::swap(e->d_state, st2);  // the loop's pointers and tensor maps take the engine's state pointers
+        std::swap(e->d_psi, psi2);
         Loop Lf;
-        std::memset(static_cast<void *>(&Lf), 0, sizeof(Lf));
-        Lf.nshots = nshots;
-        Lf.lg = launch_geo(e, nshots, false);
-        Lf.lgv = launch_geo(e, nshots, true);
+        plan_loop(e, Lf, nshots, false);
+        fill_common(e, Lf);
+        std::swap(e->d_state, st2);
+        std::swap(e->d_psi, psi2);
         int r;
         if ((r = upload_points(e, Lf.lgv, nshots, e->td_vp, &e->d_voff_t, &e->cap_voff_t, &e->d_vpts_t, &e->cap_vpts_t)) ||
             (r = upload_points(e, Lf.lg, nshots, e->td_sp, &e->d_soff_t, &e->cap_soff_t, &e->d_spts_t, &e->cap_spts_t)) ||
@@ -1397,9 +1574,6 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
         if (!e->td_amp.empty())
             CU(cudaMemcpyAsync(e->d_amp_t, e->td_amp.data(), e->td_amp.size() * sizeof(float), cudaMemcpyHostToDevice,
                                e->stream));
-        std::swap(e->d_state, st2);  // fill_common and the tensor maps take the engine's state pointers
-        std::swap(e->d_psi, psi2);
-        fill_common(e, Lf);
         Lf.va.pt_off = e->td_vp.empty() ? nullptr : e->d_voff_t;
         Lf.va.pts = e->d_vpts_t;
         Lf.va.val = e->d_amp_t;
@@ -1408,21 +1582,13 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
         Lf.sa.pts = e->d_spts_t;
         Lf.sa.amp = e->d_amp_t;
         Lf.sa.amp_row = NT;
-        {
-            const int ms = e->max_shots;  // the tensor maps cover this batch's shots only
-            e->max_shots = nshots;
-            Lf.tma = e->use_tma && setup_tma(e, Lf, nullptr);
-            e->max_shots = ms;
-        }
         std::swap(e->d_state, st2);
-        std::swap(e->d_psi, psi2);
+        r = finish_plan(e, Lf);
+        std::swap(e->d_state, st2);
+        if (r) return r;
         // the adjoint loop: the residual injected at the receivers, on the engine's state
         Loop La;
-        std::memset(static_cast<void *>(&La), 0, sizeof(La));
-        La.nshots = nshots;
-        La.back = true;
-        La.lg = launch_geo(e, nshots, false);
-        La.lgv = launch_geo(e, nshots, true);
+        plan_loop(e, La, nshots, true);
         std::vector<HostPt> va;
         for (int sh = 0; sh < nshots; ++sh)
             for (int tr = 0; tr < e->ntr; ++tr)
@@ -1434,7 +1600,7 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
         La.va.val = e->d_diff;
         La.va.val_row = e->ns;
         La.va.val_comp = (long long)e->ntr * e->ns;
-        La.tma = e->use_tma && setup_tma(e, La, nullptr);
+        if ((r = finish_plan(e, La))) return r;
         TdArgs ta;
         std::memset(static_cast<void *>(&ta), 0, sizeof(ta));  // part of the graph key, padding included
         ta.g = e->g;
@@ -1457,6 +1623,8 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
         const int nb = 2 * 148, tb = 256;
         const dim3 grd_c((p.nz + BX - 1) / BX, (p.nx + BY - 1) / BY, p.ny);
         auto integrate = [&](float *u, const float *st, float *seg) { td_integrate(e, nshots, u, st, seg, seg_shot); };
+        set_slots(Lf, 0, 0);
+        set_slots(La, 0, 0);
         auto enqueue = [&]() {
             cudaMemsetAsync(dk, 0, (size_t)4 * n * sizeof(double), e->stream);
             if (!have_ck) {
@@ -1845,11 +2013,7 @@ extern "C" int ifosb_hessian_green(ifosb_engine *e, int nrec, const int *rec_ids
         }
         float *dft = e->d_green + (long long)q0 * e->dft_shot;
         Loop L;
-        std::memset(static_cast<void *>(&L), 0, sizeof(L));  // the graph cache compares Loops bytewise
-        L.nshots = B;
-        L.back = true;
-        L.lg = launch_geo(e, B, false);
-        L.lgv = launch_geo(e, B, true);
+        plan_loop(e, L, B, true);
         if ((rc = upload_points(e, L.lgv, B, vp, &e->d_voff, &e->cap_voff, &e->d_vpts, &e->cap_vpts))) return rc;
         if ((rc = reset_state(e, B, dft))) return rc;
         fill_common(e, L);
@@ -1860,10 +2024,9 @@ extern "C" int ifosb_hessian_green(ifosb_engine *e, int nrec, const int *rec_ids
         L.va.val_comp = NT;
         L.sa.pt_off = nullptr;
         L.sa.pts = nullptr;
-        L.sa.dft = dft;
-        L.sa.trig = e->d_trig_b;
-        L.tma = e->use_tma && setup_tma(e, L, dft);
-        if ((rc = run_loop(e, L))) return rc;
+        L.dft = dft;
+        L.trig = e->d_trig_b;
+        if ((rc = finish_plan(e, L)) || (rc = run_loop(e, L))) return rc;
         if ((rc = check_unstable(e, B))) return rc;
     }
     e->ngreen = nrec;
@@ -2085,7 +2248,7 @@ extern "C" int ifosb_autotune(ifosb_engine *e, int nshots, const ifosb_shot *sho
     if (!e || !shots || nshots < 1 || nshots > e->max_shots || steps < 1) return IFOSB_EARG;
     const int saved_profile = e->profile;
     e->tuned.erase(nshots);
-    const Geo hv = launch_geo(e, nshots, true), hs = launch_geo(e, nshots, false);  // built-in choices
+    const Geo hv = box_geo(e, nshots, true), hs = box_geo(e, nshots, false);  // built-in choices
     std::vector<int> cys = {2, 3, 4, 6, 8, 12, 16, 24, 32, 64, hv.cy, hs.cy};
     {
         // chunkings whose CTA count fills one or two waves at 1-4 CTAs per SM: on
@@ -2109,8 +2272,7 @@ extern "C" int ifosb_autotune(ifosb_engine *e, int nshots, const ifosb_shot *sho
     cys.erase(std::unique(cys.begin(), cys.end()), cys.end());
     double bv = 1e30, bs = 1e30;
     const ifosb_engine::Shape *near = shape_for(e, nshots);
-    ifosb_engine::Shape pick{hv.cy, near ? near->l2v : L2AHEAD_VEL_DEFAULT, hs.cy,
-                             near ? near->l2s : L2AHEAD_STR_DEFAULT};
+    ifosb_engine::Shape pick{hv.cy, near ? near->l2v : 0, hs.cy, near ? near->l2s : 0};
     int rc = IFOSB_OK;
     e->profile = 1;
     e->nt_limit = steps;

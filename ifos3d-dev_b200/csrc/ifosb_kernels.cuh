@@ -34,7 +34,13 @@ enum { VX = 0, VY, VZ, SYY, SXY, SYZ, SXX, SZZ, SXZ, NEL };
 // first (5, or 10 with non-uniform relaxation times), then the velocity update's.
 enum { MD_PI = 0, MD_U, MD_UIPJP, MD_UJPKP, MD_UIPKP, MD_TAUS, MD_TAUP, MD_TSIPJP, MD_TSJPKP, MD_TSIPKP, MD_RIP, MD_RJP, MD_RKP, NMODEL };
 // CPML coefficient rows
-enum { K_X = 0, A_X, B_X, KH_X, AH_X, BH_X, K_Y, A_Y, B_Y, KH_Y, AH_Y, BH_Y, K_Z, A_Z, B_Z, KH_Z, AH_Z, BH_Z };
+enum { K_X = 0, A_X, B_X, KH_X, AH_X, BH_X, K_Y, A_Y, B_Y, KH_Y, AH_Y, BH_Y, K_Z, A_Z, B_Z, KH_Z, AH_Z, BH_Z,
+       RK_X, RKH_X, RK_Y, RKH_Y, NCPG };  // RK: the correctly rounded reciprocals of K
+// The z faces' coefficients per cell (index k-1; K = 1, a = b = 0 inside), so that a
+// thread reads its four cells' as one word. KS, KHS: the stress update's, which takes
+// K_y on the front face (update_s_ssg_CPML_elastic.c:104-108).
+enum { Z_K = 0, Z_RK, Z_A, Z_B, Z_KH, Z_RKH, Z_AH, Z_BH, Z_KS, Z_RKS, Z_KHS, Z_RKHS, NCZ };
+constexpr int CZ0 = NCPG * 2 * MAXFW;  // where they start; row pitch pz
 
 struct Geo {
     int nx, ny, nz, fw, free_surf, nmech;
@@ -45,6 +51,8 @@ struct Geo {
     int cy, nyc;        // y planes per block, y chunks
     int ntk, nti;       // blocks along z and x
     int by;             // rows (x) per block: the tile height of the kernels in use
+    int pzw, zfo;       // z PML slab: row pitch, and the far face's offset from k-1 (see Slabs)
+    int bz;             // cells (z) per block
 };
 
 __host__ __device__ __forceinline__ long long widx(const Geo &g, int j, int i, int k) {
@@ -59,10 +67,6 @@ struct Pt {
     int pad0, pad1, pad2;
 };
 enum { PT_EXPLOSIVE = 1, PT_ADJOINT = 6, PT_RECEIVER = 7 };
-
-__constant__ float c_cpml[18][2 * MAXFW];
-
-__device__ __forceinline__ float CP(int row, int h) { return c_cpml[row][h - 1]; }
 
 // a / b rounded to nearest (IEEE), the same bits as the division operator. The
 // division's range check sends a zero dividend down its slow path (three times
@@ -92,19 +96,22 @@ __device__ __forceinline__ int face_z(const Geo &g, int k) {
 }
 
 // PML memory slabs of a shot: 9 for the stress derivatives (velocity update),
-// then 9 for the velocity derivatives (stress update). x: [NY][2FW][NZ],
-// y: [2FW][NX][NZ], z: [NY][NX][2FW] (the reference's shapes, ifos3d.c:421-440).
+// then 9 for the velocity derivatives (stress update). x: [NY][2FW][z row],
+// y: [2FW][NX][z row], z: [NY][NX][2FW], the reference's slabs (ifos3d.c:421-440)
+// with rows padded so that the four cells a thread owns (k = 1 mod 4) are one
+// 16-byte word: x and y rows are field rows (pitch pz, k = 1 at float 8), a z row
+// holds k-1 for the near face and k-1 + zfo for the far one.
 struct Slabs {
     long long sx, sy, sz;
 };
 __device__ __forceinline__ long long sxi(const Geo &g, int j, int h, int k) {
-    return ((long long)(j - 1) * 2 * g.fw + (h - 1)) * g.nz + (k - 1);
+    return ((long long)(j - 1) * 2 * g.fw + (h - 1)) * g.pz + (k + 7);
 }
 __device__ __forceinline__ long long syi(const Geo &g, int h, int i, int k) {
-    return ((long long)(h - 1) * g.nx + (i - 1)) * g.nz + (k - 1);
+    return ((long long)(h - 1) * g.nx + (i - 1)) * g.pz + (k + 7);
 }
 __device__ __forceinline__ long long szi(const Geo &g, int j, int i, int h) {
-    return ((long long)(j - 1) * g.nx + (i - 1)) * 2 * g.fw + (h - 1);
+    return ((long long)(j - 1) * g.nx + (i - 1)) * g.pzw + (h <= g.fw ? h - 1 : h - 1 - 2 * g.fw + g.nz + g.zfo);
 }
 
 struct VelArgs {
@@ -112,7 +119,11 @@ struct VelArgs {
     Slabs sl;
     float *st;            // state base (shot 0)
     long long st_shot;    // floats per shot
+    const float *vin;     // velocities before the step [shot][3][field], and where the new ones go
+    float *vout;          // (a slot of the velocity ring; the same place without one)
+    long long vin_shot, vout_shot;
     const float *md;      // model base
+    const float *rho;     // rho in field layout (with matcopy's ghost layers)
     float *psi;           // PML memory base (shot 0)
     long long psi_shot;
     const int *pt_off;    // [nshots][nblocks+1] or null
@@ -123,6 +134,7 @@ struct VelArgs {
     float b1, b2;
     double cf5x, cf5y, cf5z;  // type-5 force direction factors (update_v_ssg.c:498-503)
     const float *cpg;         // global copy of the CPML rows, for lane-divergent (z-face) reads
+    int fast_div;         // every density and CPML divisor is in div4's range
     int *err_step;        // [nshots] first step whose probe cell went NaN
     int probe_j, probe_i, probe_k;
 };
@@ -141,10 +153,8 @@ struct StrArgs {
     long long amp_row;
     float *sec;           // traces [shot][3][ntr][ns]
     long long sec_shot, sec_comp, sec_tr;
-    float *dft;           // [shot][nf][6][field]
-    long long dft_shot;
-    int nf;
-    const double *trig;   // [NT][nf][2]: cos, sin of 2 pi f t, times DT*ntast
+    const float *v;       // velocities of this step [shot][3][field]
+    long long v_shot;
     float dt, dthalbe, rdx, rdy, rdz;
     float b1, b2;
     float eta[MAXMECH], mb[MAXMECH], mc[MAXMECH], msb[MAXMECH];
@@ -152,6 +162,10 @@ struct StrArgs {
     int seismo;           // SEISMO: 1 particle velocities; 2, 3, 4 add p / div, curl (sec2)
     float *sec2;          // [shot][3][ntr][ns]: p, div, curl
     float hrx, hry, hrz;  // 1.0/DX etc. in float (seismo_ssg.c:38-40)
+    int fast_div;         // every CPML divisor and spacing is in div4's range
+    int unif_tau;         // one relaxation time for all cells (utaus, utaup and the average)
+    float utaus, utaup, uts_avg;
+    float idx, idy, idz;  // RN(1/DX) etc. (exact for power-of-two spacings)
     const float *smod;    // elastic free surface: pi, u of plane j=1 ([2][NX][NZ]) when they
                           // differ from the propagation model's, else null
 };
@@ -188,357 +202,52 @@ __device__ __forceinline__ void block_points(const int *pt_off, const Geo &g, in
 }
 
 // ---------------------------------------------------------------------------
-// Velocity update: update_v_ssg.c:102-127, update_v_ssg_CPML.c, and the point
-// forces of update_v_ssg.c:474-522 / update_v_ssg_CPML.c:384-393.
-template <bool BACK>
-__device__ __forceinline__ void vel_points(const VelArgs &a, float *st, int p0, int p1, int j, int i, int k, int nt,
-                                           long long c) {
-    const long long F = a.g.field;
-    for (int q = p0; q < p1; ++q) {
-        const Pt pt = a.pts[q];
-        if (pt.j != j || pt.i != i || pt.k != k) continue;
-        if (BACK) {
-            const float *v = a.val + (long long)pt.row * a.val_row + (nt - 1);
-            st[VX * F + c] += v[0];
-            st[VZ * F + c] += v[2 * a.val_comp];
-            st[VY * F + c] += v[a.val_comp];
-        } else {
-            const float amp = a.val[(long long)pt.row * a.val_row + (nt - 1)];
-            switch (pt.kind) {
-            case 2: st[VX * F + c] += amp * a.md[MD_RIP * F + c]; break;
-            case 3: st[VZ * F + c] += amp * a.md[MD_RJP * F + c]; break;  // rjp for vz as in the reference
-            case 4: st[VY * F + c] += amp * a.md[MD_RKP * F + c]; break;  // rkp for vy as in the reference
-            case 5:
-                st[VX * F + c] = (float)((double)st[VX * F + c] + a.cf5x * (double)amp);
-                st[VY * F + c] = (float)((double)st[VY * F + c] + a.cf5y * (double)amp);
-                st[VZ * F + c] = (float)((double)st[VZ * F + c] + a.cf5z * (double)amp);
-                break;
-            default: break;
-            }
-        }
-    }
-}
-
-template <bool BACK>
-__global__ void __launch_bounds__(BX *BY) k_velocity(VelArgs a, int nt) {
+// discfourier (disc_fourier.c:36-57) for P steps at once: every accumulator takes the
+// steps' velocities in order, F += v * trig with product and sum in double and a float
+// store each time, so the bits are those of one pass per step. A pass reads and writes
+// the 6 nf accumulators of a cell (48 nf bytes), which at one pass a step is more than
+// a third of an L = 3, nf = 4 step's traffic; over P steps it costs 12 + 48 nf / P
+// bytes a step, the 12 being the velocities, kept in a ring for it.
+constexpr int MAXRING = 8;
+struct DftArgs {
+    Geo g;
+    const float *v[MAXRING];  // velocities of the steps [shot][3][field]
+    long long v_shot[MAXRING];
+    const double *trig[MAXRING];  // cos, sin of 2 pi f t, times DT*ntast, [nf][2] of each step
+    float *dft;               // [shot][nf][6][field]
+    long long dft_shot;
+    int nf;
+};
+// One velocity component (blockIdx.y) of four z-adjacent cells a thread.
+template <int P>
+__global__ void __launch_bounds__(128) k_dft(const __grid_constant__ DftArgs a) {
     const Geo &g = a.g;
-    const int k = blockIdx.x * BX + threadIdx.x + 1;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y + 1;  // blockDim.y == g.by
-    const int yc = blockIdx.z % g.nyc, s = blockIdx.z / g.nyc;
-    int p0, p1;
-    block_points(a.pt_off, g, s, yc, p0, p1);
-    if (k > g.nz || i > g.nx) return;
-    const int j0 = yc * g.cy + 1;
-    const int j1 = min(j0 + g.cy - 1, g.ny);
-    float *st = a.st + (long long)s * a.st_shot;
-    float *ps = a.psi + (long long)s * a.psi_shot;
-    const long long F = g.field;
-    const float *__restrict__ sxx = st + SXX * F;
-    const float *__restrict__ syy = st + SYY * F;
-    const float *__restrict__ szz = st + SZZ * F;
-    const float *__restrict__ sxy = st + SXY * F;
-    const float *__restrict__ syz = st + SYZ * F;
-    const float *__restrict__ sxz = st + SXZ * F;
-    const float b1 = a.b1, b2 = a.b2, dx = a.dxr, dy = a.dyr, dz = a.dzr;
-    const long long dI = g.pz, dJ = g.plane;
-    const int hx = face_x(g, i), hz = face_z(g, k);
-    for (int j = j0; j <= j1; ++j) {
-        const long long c = widx(g, j, i, k);
-        float sxx_x = dx * (b1 * (__ldg(sxx + c + dI) - __ldg(sxx + c)) + b2 * (__ldg(sxx + c + 2 * dI) - __ldg(sxx + c - dI)));
-        float sxy_y = dy * (b1 * (__ldg(sxy + c) - __ldg(sxy + c - dJ)) + b2 * (__ldg(sxy + c + dJ) - __ldg(sxy + c - 2 * dJ)));
-        float sxz_z = dz * (b1 * (__ldg(sxz + c) - __ldg(sxz + c - 1)) + b2 * (__ldg(sxz + c + 1) - __ldg(sxz + c - 2)));
-        float syy_y = dy * (b1 * (__ldg(syy + c + dJ) - __ldg(syy + c)) + b2 * (__ldg(syy + c + 2 * dJ) - __ldg(syy + c - dJ)));
-        float sxy_x = dx * (b1 * (__ldg(sxy + c) - __ldg(sxy + c - dI)) + b2 * (__ldg(sxy + c + dI) - __ldg(sxy + c - 2 * dI)));
-        float syz_z = dz * (b1 * (__ldg(syz + c) - __ldg(syz + c - 1)) + b2 * (__ldg(syz + c + 1) - __ldg(syz + c - 2)));
-        float szz_z = dz * (b1 * (__ldg(szz + c + 1) - __ldg(szz + c)) + b2 * (__ldg(szz + c + 2) - __ldg(szz + c - 1)));
-        float sxz_x = dx * (b1 * (__ldg(sxz + c) - __ldg(sxz + c - dI)) + b2 * (__ldg(sxz + c + dI) - __ldg(sxz + c - 2 * dI)));
-        float syz_y = dy * (b1 * (__ldg(syz + c) - __ldg(syz + c - dJ)) + b2 * (__ldg(syz + c + dJ) - __ldg(syz + c - 2 * dJ)));
-        const int hy = face_y(g, j);
-        const bool frame = hx || hy || hz;
-        if (hx) {
-            float *p = ps + sxi(g, j, hx, k);
-            const long long o = a.sl.sx;
-            float v0 = CP(BH_X, hx) * p[0] + CP(AH_X, hx) * sxx_x; p[0] = v0; sxx_x = sxx_x / CP(KH_X, hx) + v0;
-            float v1 = CP(B_X, hx) * p[o] + CP(A_X, hx) * sxy_x; p[o] = v1; sxy_x = sxy_x / CP(K_X, hx) + v1;
-            float v2 = CP(B_X, hx) * p[2 * o] + CP(A_X, hx) * sxz_x; p[2 * o] = v2; sxz_x = sxz_x / CP(K_X, hx) + v2;
+    const int nq = (g.nz + 3) / 4, id = blockIdx.x * blockDim.x + threadIdx.x, row = id / nq;
+    const int j = row / g.nx + 1, i = row % g.nx + 1, k = 4 * (id % nq) + 1, c = blockIdx.y, s = blockIdx.z;
+    if (j > g.ny) return;
+    const long long F = g.field, at = (long long)c * F + widx(g, j, i, k);
+    float4 v[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) v[p] = __ldg(reinterpret_cast<const float4 *>(a.v[p] + (long long)s * a.v_shot[p] + at));
+    float *f = a.dft + (long long)s * a.dft_shot + at;
+    const int n = g.nz - k + 1;
+    for (int l = 0; l < 2 * a.nf; ++l, f += 3 * F) {  // cos and sin accumulators in turn
+        const float4 o = *reinterpret_cast<const float4 *>(f);
+        float x[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+            const double t = a.trig[p][l];
+            x[0] = (float)((double)x[0] + (double)v[p].x * t);
+            x[1] = (float)((double)x[1] + (double)v[p].y * t);
+            x[2] = (float)((double)x[2] + (double)v[p].z * t);
+            x[3] = (float)((double)x[3] + (double)v[p].w * t);
         }
-        if (hy) {
-            float *p = ps + 3 * a.sl.sx + syi(g, hy, i, k);
-            const long long o = a.sl.sy;
-            float v0 = CP(B_Y, hy) * p[0] + CP(A_Y, hy) * sxy_y; p[0] = v0; sxy_y = sxy_y / CP(K_Y, hy) + v0;
-            float v1 = CP(BH_Y, hy) * p[o] + CP(AH_Y, hy) * syy_y; p[o] = v1; syy_y = syy_y / CP(KH_Y, hy) + v1;
-            float v2 = CP(B_Y, hy) * p[2 * o] + CP(A_Y, hy) * syz_y; p[2 * o] = v2; syz_y = syz_y / CP(K_Y, hy) + v2;
-        }
-        if (hz) {
-            float *p = ps + 3 * a.sl.sx + 3 * a.sl.sy + szi(g, j, i, hz);
-            const long long o = a.sl.sz;
-            float v0 = CP(B_Z, hz) * p[0] + CP(A_Z, hz) * sxz_z; p[0] = v0; sxz_z = sxz_z / CP(K_Z, hz) + v0;
-            float v1 = CP(B_Z, hz) * p[o] + CP(A_Z, hz) * syz_z; p[o] = v1; syz_z = syz_z / CP(K_Z, hz) + v1;
-            float v2 = CP(BH_Z, hz) * p[2 * o] + CP(AH_Z, hz) * szz_z; p[2 * o] = v2; szz_z = szz_z / CP(KH_Z, hz) + v2;
-        }
-        // CPML frame: update_v() applies its point forces before update_v_CPML() updates the frame
-        if (frame && p1 > p0) vel_points<BACK>(a, st, p0, p1, j, i, k, nt, c);
-        st[VX * F + c] += (sxx_x + sxy_y + sxz_z) / a.md[MD_RIP * F + c];
-        st[VY * F + c] += (syy_y + sxy_x + syz_z) / a.md[MD_RJP * F + c];
-        st[VZ * F + c] += (szz_z + sxz_x + syz_y) / a.md[MD_RKP * F + c];
-        if (p1 > p0) {
-            // interior: forces after the update (the adjoint injects twice);
-            // frame: only the adjoint's second injection (update_v_ssg_CPML.c:384-393)
-            const int passes = frame ? (BACK ? 1 : 0) : (BACK ? 2 : 1);
-            for (int pass = 0; pass < passes; ++pass) vel_points<BACK>(a, st, p0, p1, j, i, k, nt, c);
-        }
-        if (j == a.probe_j && i == a.probe_i && k == a.probe_k) {
-            if (isnan(st[VY * F + c])) atomicMin(a.err_step + s, nt);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Stress update and the rest of the time step, per cell, in the reference's order:
-//   1. update_s_elastic / update_s (L mechanisms) with the CPML psi recursions
-//      (update_s_ssg_elastic.c:106-140, update_s_ssg.c:150-230,
-//       update_s_ssg_CPML(_elastic).c)
-//   2. psource (psource.c:38-52)
-//   3. discfourier (disc_fourier.c:36-57)
-//   4. surface_elastic / surface at j=1 (surface_ssg_elastic.c:69-111,
-//      surface_ssg.c:117-160), mirror rows j=0,-1 written by the j=1..3 cells
-//   5. seismo (seismo_ssg.c:43-50)
-template <int L>
-__global__ void __launch_bounds__(BX *BY) k_stress(StrArgs a, int nt, int do_dft, int sample) {
-    const Geo &g = a.g;
-    const int k = blockIdx.x * BX + threadIdx.x + 1;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y + 1;  // blockDim.y == g.by
-    const int yc = blockIdx.z % g.nyc, s = blockIdx.z / g.nyc;
-    int p0, p1;
-    block_points(a.pt_off, g, s, yc, p0, p1);
-    if (k > g.nz || i > g.nx) return;
-    const int j0 = yc * g.cy + 1;
-    const int j1 = min(j0 + g.cy - 1, g.ny);
-    float *st = a.st + (long long)s * a.st_shot;
-    float *ps = a.psi + (long long)s * a.psi_shot + 3 * (a.sl.sx + a.sl.sy + a.sl.sz);
-    const long long F = g.field;
-    const float *__restrict__ vx = st + VX * F;
-    const float *__restrict__ vy = st + VY * F;
-    const float *__restrict__ vz = st + VZ * F;
-    const float b1 = a.b1, b2 = a.b2, DX = a.rdx, DY = a.rdy, DZ = a.rdz, DT = a.dt;
-    const long long dI = g.pz, dJ = g.plane;
-    const int hx = face_x(g, i), hz = face_z(g, k);
-    const bool zfront = k <= g.fw;
-    for (int j = j0; j <= j1; ++j) {
-        const long long c = widx(g, j, i, k);
-        const float vx0 = __ldg(vx + c), vy0 = __ldg(vy + c), vz0 = __ldg(vz + c);
-        float vxx = (b1 * (vx0 - __ldg(vx + c - dI)) + b2 * (__ldg(vx + c + dI) - __ldg(vx + c - 2 * dI))) / DX;
-        float vxy = (b1 * (__ldg(vx + c + dJ) - vx0) + b2 * (__ldg(vx + c + 2 * dJ) - __ldg(vx + c - dJ))) / DY;
-        float vxz = (b1 * (__ldg(vx + c + 1) - vx0) + b2 * (__ldg(vx + c + 2) - __ldg(vx + c - 1))) / DZ;
-        float vyx = (b1 * (__ldg(vy + c + dI) - vy0) + b2 * (__ldg(vy + c + 2 * dI) - __ldg(vy + c - dI))) / DX;
-        float vyy = (b1 * (vy0 - __ldg(vy + c - dJ)) + b2 * (__ldg(vy + c + dJ) - __ldg(vy + c - 2 * dJ))) / DY;
-        float vyz = (b1 * (__ldg(vy + c + 1) - vy0) + b2 * (__ldg(vy + c + 2) - __ldg(vy + c - 1))) / DZ;
-        float vzx = (b1 * (__ldg(vz + c + dI) - vz0) + b2 * (__ldg(vz + c + 2 * dI) - __ldg(vz + c - dI))) / DX;
-        float vzy = (b1 * (__ldg(vz + c + dJ) - vz0) + b2 * (__ldg(vz + c + 2 * dJ) - __ldg(vz + c - dJ))) / DY;
-        float vzz = (b1 * (vz0 - __ldg(vz + c - 1)) + b2 * (__ldg(vz + c + 1) - __ldg(vz + c - 2))) / DZ;
-        // the free surface works on the plain derivatives (surface_ssg_elastic.c:91-93)
-        const float svxx = vxx, svyy = vyy, svzz = vzz;
-        const int hy = face_y(g, j);
-        if (hx) {
-            float *p = ps + sxi(g, j, hx, k);
-            const long long o = a.sl.sx;
-            float v0 = CP(B_X, hx) * p[0] + CP(A_X, hx) * vxx; p[0] = v0; vxx = vxx / CP(K_X, hx) + v0;
-            float v1 = CP(BH_X, hx) * p[o] + CP(AH_X, hx) * vyx; p[o] = v1; vyx = vyx / CP(KH_X, hx) + v1;
-            float v2 = CP(BH_X, hx) * p[2 * o] + CP(AH_X, hx) * vzx; p[2 * o] = v2; vzx = vzx / CP(KH_X, hx) + v2;
-        }
-        if (hy) {
-            float *p = ps + 3 * a.sl.sx + syi(g, hy, i, k);
-            const long long o = a.sl.sy;
-            float v0 = CP(BH_Y, hy) * p[0] + CP(AH_Y, hy) * vxy; p[0] = v0; vxy = vxy / CP(KH_Y, hy) + v0;
-            float v1 = CP(B_Y, hy) * p[o] + CP(A_Y, hy) * vyy; p[o] = v1; vyy = vyy / CP(K_Y, hy) + v1;
-            float v2 = CP(BH_Y, hy) * p[2 * o] + CP(AH_Y, hy) * vzy; p[2 * o] = v2; vzy = vzy / CP(KH_Y, hy) + v2;
-        }
-        if (hz) {
-            // the reference divides by K_y on the front z face (update_s_ssg_CPML_elastic.c:104-108)
-            float *p = ps + 3 * a.sl.sx + 3 * a.sl.sy + szi(g, j, i, hz);
-            const long long o = a.sl.sz;
-            const float kh = zfront ? CP(KH_Y, hz) : CP(KH_Z, hz);
-            const float kf = zfront ? CP(K_Y, hz) : CP(K_Z, hz);
-            float v0 = CP(BH_Z, hz) * p[0] + CP(AH_Z, hz) * vxz; p[0] = v0; vxz = vxz / kh + v0;
-            float v1 = CP(BH_Z, hz) * p[o] + CP(AH_Z, hz) * vyz; p[o] = v1; vyz = vyz / kh + v1;
-            float v2 = CP(B_Z, hz) * p[2 * o] + CP(A_Z, hz) * vzz; p[2 * o] = v2; vzz = vzz / kf + v2;
-        }
-        const float *md = a.md;
-        const float uipjp = md[MD_UIPJP * F + c], ujpkp = md[MD_UJPKP * F + c], uipkp = md[MD_UIPKP * F + c];
-        const float pim = md[MD_PI * F + c], um = md[MD_U * F + c];
-        const float vxyyx = vxy + vyx, vyzzy = vyz + vzy, vxzzx = vxz + vzx;
-        const float vxxyyzz = vxx + vyy + vzz, vyyzz = vyy + vzz, vxxzz = vxx + vzz, vxxyy = vxx + vyy;
-        float *S = st + c;
-        float sxx = S[SXX * F], syy = S[SYY * F], szz = S[SZZ * F], sxy = S[SXY * F], syz = S[SYZ * F], sxz = S[SXZ * F];
-        // ---- 1. stress (and memory variables) -----------------------------------
-        float rv[L > 0 ? L : 1][6];
-        float taus = 0.f, taup = 0.f;
-        if constexpr (L == 0) {
-            const float fipjp = uipjp * DT, fjpkp = ujpkp * DT, fipkp = uipkp * DT;
-            const float gg = pim, f = (float)(2.0 * (double)um);
-            sxy += (fipjp * vxyyx);
-            syz += (fjpkp * vyzzy);
-            sxz += (fipkp * vxzzx);
-            sxx += DT * ((gg * vxxyyzz) - (f * vyyzz));
-            syy += DT * ((gg * vxxyyzz) - (f * vxxzz));
-            szz += DT * ((gg * vxxyyzz) - (f * vxxyy));
+        if (n >= 4) {
+            *reinterpret_cast<float4 *>(f) = make_float4(x[0], x[1], x[2], x[3]);
         } else {
-            const float tausipjp = md[MD_TSIPJP * F + c], tausjpkp = md[MD_TSJPKP * F + c], tausipkp = md[MD_TSIPKP * F + c];
-            taus = md[MD_TAUS * F + c];
-            taup = md[MD_TAUP * F + c];
-            const float Lf = (float)L, dthalbe = a.dthalbe;
-            const float *r = st + NEL * F + c;
-            float sr[6];
 #pragma unroll
-            for (int l = 0; l < L; ++l)
-#pragma unroll
-                for (int q = 0; q < 6; ++q) rv[l][q] = r[(6 * l + q) * F];
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                sr[q] = rv[0][q];
-#pragma unroll
-                for (int l = 1; l < L; ++l) sr[q] += rv[l][q];
-            }
-            const float fipjp = (float)((double)(uipjp * DT) * (1.0 + (double)(Lf * tausipjp)));
-            const float fjpkp = (float)((double)(ujpkp * DT) * (1.0 + (double)(Lf * tausjpkp)));
-            const float fipkp = (float)((double)(uipkp * DT) * (1.0 + (double)(Lf * tausipkp)));
-            const float gg = (float)((double)pim * (1.0 + (double)(Lf * taup)));
-            const float f = (float)((2.0 * (double)um) * (1.0 + (double)(Lf * taus)));
-            sxy += (fipjp * vxyyx) + (dthalbe * sr[3]);
-            syz += (fjpkp * vyzzy) + (dthalbe * sr[4]);
-            sxz += (fipkp * vxzzx) + (dthalbe * sr[5]);
-            sxx += DT * ((gg * vxxyyzz) - (f * vyyzz)) + (dthalbe * sr[0]);
-            syy += DT * ((gg * vxxyyzz) - (f * vxxzz)) + (dthalbe * sr[1]);
-            szz += DT * ((gg * vxxyyzz) - (f * vxxyy)) + (dthalbe * sr[2]);
-#pragma unroll
-            for (int l = 0; l < L; ++l) {
-                const float eta = a.eta[l], bb = a.mb[l], cc = a.mc[l];
-                const float dipjp = uipjp * eta * tausipjp, djpkp = ujpkp * eta * tausjpkp, dipkp = uipkp * eta * tausipkp;
-                const float d = (float)(((2.0 * (double)um) * (double)eta) * (double)taus);
-                const float e = pim * eta * taup;
-                rv[l][3] = bb * (rv[l][3] * cc - (dipjp * vxyyx));
-                rv[l][4] = bb * (rv[l][4] * cc - (djpkp * vyzzy));
-                rv[l][5] = bb * (rv[l][5] * cc - (dipkp * vxzzx));
-                rv[l][0] = bb * (rv[l][0] * cc - (e * vxxyyzz) + (d * vyyzz));
-                rv[l][1] = bb * (rv[l][1] * cc - (e * vxxyyzz) + (d * vxxzz));
-                rv[l][2] = bb * (rv[l][2] * cc - (e * vxxyyzz) + (d * vxxyy));
-            }
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                sr[q] = rv[0][q];
-#pragma unroll
-                for (int l = 1; l < L; ++l) sr[q] += rv[l][q];
-            }
-            sxy += (dthalbe * sr[3]);
-            syz += (dthalbe * sr[4]);
-            sxz += (dthalbe * sr[5]);
-            sxx += (dthalbe * sr[0]);
-            syy += (dthalbe * sr[1]);
-            szz += (dthalbe * sr[2]);
-        }
-        // ---- 2. explosive sources ------------------------------------------------
-        for (int q = p0; q < p1; ++q) {
-            const Pt pt = a.pts[q];
-            if (pt.kind == PT_EXPLOSIVE && pt.j == j && pt.i == i && pt.k == k) {
-                const float amp = a.amp[(long long)pt.row * a.amp_row + (nt - 1)];
-                sxx += amp; syy += amp; szz += amp;
-            }
-        }
-        // ---- 3. on-the-fly DFT of the velocities ----------------------------------
-        if (do_dft) {
-            float *Fd = a.dft + (long long)s * a.dft_shot + c;
-            const double *tr = a.trig + (long long)(nt - 1) * a.nf * 2;
-            for (int l = 0; l < a.nf; ++l) {
-                const double t1 = tr[2 * l], t2 = tr[2 * l + 1];
-                float *Fl = Fd + (long long)l * 6 * F;
-                Fl[0 * F] = (float)((double)Fl[0 * F] + (double)vx0 * t1);
-                Fl[1 * F] = (float)((double)Fl[1 * F] + (double)vy0 * t1);
-                Fl[2 * F] = (float)((double)Fl[2 * F] + (double)vz0 * t1);
-                Fl[3 * F] = (float)((double)Fl[3 * F] + (double)vx0 * t2);
-                Fl[4 * F] = (float)((double)Fl[4 * F] + (double)vy0 * t2);
-                Fl[5 * F] = (float)((double)Fl[5 * F] + (double)vz0 * t2);
-            }
-        }
-        // ---- 4. free surface ---------------------------------------------------
-        if (g.free_surf && j == 1) {
-            syy = 0.0f;
-            if constexpr (L == 0) {
-                float spi = pim, su = um;
-                if (a.smod) {
-                    const long long q = (long long)(i - 1) * g.nz + (k - 1);
-                    spi = a.smod[q];
-                    su = a.smod[(long long)g.nx * g.nz + q];
-                }
-                const float f = (float)((double)su * 2.0), gg = spi;
-                const float h = -(DT * (gg - f) * (gg - f) * (svxx + svzz) / gg) - (DT * (gg - f) * svyy);
-                sxx += h;
-                szz += h;
-            } else {
-                const float Lf = (float)L, dthalbe = a.dthalbe;
-#pragma unroll
-                for (int l = 0; l < L; ++l) rv[l][1] = 0.0f;
-                const float f = (float)(((double)um * 2.0) * (1.0 + (double)(Lf * taus)));
-                const float gg = (float)((double)pim * (1.0 + (double)(Lf * taup)));
-                const float h = -(DT * (gg - f) * (gg - f) * (svxx + svzz) / gg) - (DT * (gg - f) * svyy);
-                float srx = rv[0][0], srz = rv[0][2];
-#pragma unroll
-                for (int l = 1; l < L; ++l) { srx += rv[l][0]; srz += rv[l][2]; }
-                sxx += h - (dthalbe * srx);
-                szz += h - (dthalbe * srz);
-                const float d = (float)((2.0 * (double)um) * (double)taus);
-                const float e = pim * taup;
-#pragma unroll
-                for (int l = 0; l < L; ++l) {
-                    const float hh = (float)((double)a.msb[l] *
-                                             ((((double)(d - e) * ((double)(f / gg) - 1.0)) * (double)(svxx + svzz)) -
-                                              (double)((d - e) * svyy)));
-                    rv[l][0] += hh;
-                    rv[l][2] += hh;
-                }
-                srx = rv[0][0]; srz = rv[0][2];
-#pragma unroll
-                for (int l = 1; l < L; ++l) { srx += rv[l][0]; srz += rv[l][2]; }
-                sxx += (dthalbe * srx);
-                szz += (dthalbe * srz);
-            }
-        }
-        S[SXX * F] = sxx; S[SYY * F] = syy; S[SZZ * F] = szz;
-        S[SXY * F] = sxy; S[SYZ * F] = syz; S[SXZ * F] = sxz;
-        if constexpr (L > 0) {
-            float *r = st + NEL * F + c;
-#pragma unroll
-            for (int l = 0; l < L; ++l)
-#pragma unroll
-                for (int q = 0; q < 6; ++q) r[(6 * l + q) * F] = rv[l][q];
-        }
-        if (g.free_surf && j <= 3) {
-            // image rows above the surface (surface_ssg_elastic.c:80-84)
-            if (j == 1) { S[SXY * F - dJ] = -sxy; S[SYZ * F - dJ] = -syz; }
-            if (j == 2) { S[SYY * F - 2 * dJ] = -syy; S[SXY * F - 3 * dJ] = -sxy; S[SYZ * F - 3 * dJ] = -syz; }
-            if (j == 3) { S[SYY * F - 4 * dJ] = -syy; }
-        }
-        // ---- 5. receivers --------------------------------------------------------
-        if (sample >= 0) {
-            for (int q = p0; q < p1; ++q) {
-                const Pt pt = a.pts[q];
-                if (pt.kind == PT_RECEIVER && pt.j == j && pt.i == i && pt.k == k) {
-                    float *o = a.sec + (long long)s * a.sec_shot + (long long)pt.row * a.sec_tr + sample;
-                    o[0] = vx0;
-                    o[a.sec_comp] = vy0;
-                    o[2 * a.sec_comp] = vz0;
-                    if (a.seismo >= 2) {
-                        float pr, dv, cu;
-                        seismo_pdc(vx0, __ldg(vx + c - dI), __ldg(vx + c + dJ), __ldg(vx + c + 1), vy0, __ldg(vy + c - dJ),
-                                   __ldg(vy + c + dI), __ldg(vy + c + 1), vz0, __ldg(vz + c - 1), __ldg(vz + c + dI),
-                                   __ldg(vz + c + dJ), sxx, syy, szz, a.md[MD_PI * F + c], a.md[MD_U * F + c], a.hrx,
-                                   a.hry, a.hrz, pr, dv, cu);
-                        float *o2 = a.sec2 + (long long)s * a.sec_shot + (long long)pt.row * a.sec_tr + sample;
-                        o2[0] = pr;
-                        o2[a.sec_comp] = dv;
-                        o2[2 * a.sec_comp] = cu;
-                    }
-                }
-            }
+            for (int q = 0; q < 3; ++q)
+                if (q < n) f[q] = x[q];
         }
     }
 }
