@@ -5,9 +5,9 @@
 // reads from the wavefield and the model: each field with just the halo its
 // derivatives need, every box completing on one mbarrier. The other threads fetch
 // their PML memories meanwhile; then the whole update runs out of shared memory and the
-// results go straight to HBM as 16-byte words. Nothing waits inside the update, so two
-// or three CTAs per SM keep 100 KB and more of loads in flight, which is what the
-// step needs: it moves 2 to 3 bytes per flop.
+// results go straight to HBM as 16-byte words. Nothing waits inside the update, so four
+// CTAs per SM keep 100 KB and more of loads in flight, which is what the step needs: it
+// moves 2 to 3 bytes per flop.
 //
 // Why boxes: a version that streamed along y through a six-plane ring (one plane of
 // loads in flight behind a producer warp, one cell per thread) spent its time waiting
@@ -98,9 +98,13 @@ struct StrBox {
     WaitCtl w;
 };
 
-constexpr int VYB = 4;  // planes of a velocity box: 62 KB, three CTAs per SM
-// planes of a stress box: 82 KB elastic; 86 KB with L = 3 (two CTAs per SM either way)
-__host__ __device__ constexpr int str_yb(int nmech) { return nmech == 0 ? 4 : 2; }
+// Planes of a box. Four CTAs per SM (16 warps, 8 with mechanisms) that are each at another
+// point of their load-update-store sequence beat two larger ones, although the y halo is
+// then read from L2 more often: velocity 2 planes (38 KB) 218 us at 256^3, 4 planes 243;
+// elastic stress with the DFT at 128^3 2 planes (49 KB) 66.7 us, 4 planes 69.5; L = 3
+// stress 1 plane (51 KB) 730 us at 256^3, 2 planes 738.
+constexpr int VYB = 2;
+__host__ __device__ constexpr int str_yb(int nmech) { return nmech == 0 ? 2 : 1; }
 
 // This thread's cells in a CTA's box, and the chunk's planes.
 struct BoxAt {
@@ -159,7 +163,7 @@ __device__ __forceinline__ void box_loop(uint64_t *full, int *err, WaitCtl w, in
 }
 
 template <bool BACK>
-__global__ void __launch_bounds__(64 * VYB, 2) k_velocity_box(const __grid_constant__ VelBox T, int nt) {
+__global__ void __launch_bounds__(64 * VYB, 4) k_velocity_box(const __grid_constant__ VelBox T, int nt) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full;
     using M = VelSm<VYB>;
@@ -197,12 +201,12 @@ __global__ void __launch_bounds__(64 * VYB, 2) k_velocity_box(const __grid_const
             tma_prefetch5(&T.v, z, x, y, VX, s);
             tma_prefetch3(&T.rho, z, x, y);
         },
-        [&](int j) { psi_load(q, g, a.sl, ps, j, b.i, b.k); },
+        [&](int j) { psi_find(q, g, a.sl, ps, j, b.i, b.k); },
         [&](int j) { vel_quad<BACK>(a, M(sm, b.y, b.x, b.zq), q, nt, s, j, b.i, b.k, g.nz - b.k + 1, p0, p1); });
 }
 
 template <int L, bool P2>
-__global__ void __launch_bounds__(64 * str_yb(L), 2) k_stress_box(const __grid_constant__ StrBox T, int nt, int sample) {
+__global__ void __launch_bounds__(64 * str_yb(L), 4) k_stress_box(const __grid_constant__ StrBox T, int nt, int sample) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint64_t full;
     constexpr int YB = str_yb(L);
@@ -235,7 +239,7 @@ __global__ void __launch_bounds__(64 * str_yb(L), 2) k_stress_box(const __grid_c
             tma_prefetch5(&T.sr, z, x, y, SYY, s);
             tma_prefetch4(&T.mod, z, x, y, 0);
         },
-        [&](int j) { psi_load(q, g, a.sl, ps, j, b.i, b.k); },
+        [&](int j) { psi_find(q, g, a.sl, ps, j, b.i, b.k); },
         [&](int j) {
             str_quad<L, P2>(a, M(sm, T.nsr, b.y, b.x, b.zq), q, nt, sample, s, j, b.i, b.k, g.nz - b.k + 1, p0, p1);
         });

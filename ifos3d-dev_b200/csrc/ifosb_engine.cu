@@ -215,7 +215,7 @@ static int dgrow(ifosb_engine *e, T **ptr, size_t *cap, size_t count) {
     return rc;
 }
 
-static bool div_range(float b) { return fabsf(b) >= DIV_B_MIN && fabsf(b) <= DIV_B_MAX; }
+static bool div_range(float b) { return b >= DIV_B_MIN && b <= DIV_B_MAX; }
 
 static void fd_coeffs(int fdcoeff, float *b1, float *b2) {
     *b1 = 9.0 / 8.0; *b2 = -1.0 / 24.0;                  // Taylor (update_v_ssg.c:97)
@@ -475,16 +475,16 @@ extern "C" int ifosb_set_cpml(ifosb_engine *e, const float *coeff) {
         for (int h = 0; h < n2; ++h) e->cpml_div = e->cpml_div && div_range(row(r, h));
     for (int h = 0; h < n2; ++h) {
         const int src[4] = {K_X, KH_X, K_Y, KH_Y}, dst[4] = {RK_X, RKH_X, RK_Y, RKH_Y};
-        for (int q = 0; q < 4; ++q) host[(size_t)dst[q] * 2 * MAXFW + h] = 1.0f / row(src[q], h);
+        for (int q = 0; q < 4; ++q) host[(size_t)dst[q] * 2 * MAXFW + h] = -1.0f / row(src[q], h);
     }
     for (int k = 1; k <= pz; ++k) {
         const int h = k <= fw ? k : (k > nz - fw && k <= nz ? k - nz + n2 : 0);
         float *c = host.data() + CZ0 + (k - 1);
         const float kf = h ? row(K_Z, h - 1) : 1.f, kh = h ? row(KH_Z, h - 1) : 1.f;
         const float sf = h && k <= fw ? row(K_Y, h - 1) : kf, sh = h && k <= fw ? row(KH_Y, h - 1) : kh;
-        const float v[NCZ] = {kf, 1.0f / kf, h ? row(A_Z, h - 1) : 0.f, h ? row(B_Z, h - 1) : 0.f,
-                              kh, 1.0f / kh, h ? row(AH_Z, h - 1) : 0.f, h ? row(BH_Z, h - 1) : 0.f,
-                              sf, 1.0f / sf, sh, 1.0f / sh};
+        const float v[NCZ] = {kf, -1.0f / kf, h ? row(A_Z, h - 1) : 0.f, h ? row(B_Z, h - 1) : 0.f,
+                              kh, -1.0f / kh, h ? row(AH_Z, h - 1) : 0.f, h ? row(BH_Z, h - 1) : 0.f,
+                              sf, -1.0f / sf, sh, -1.0f / sh};
         for (int q = 0; q < NCZ; ++q) c[(size_t)q * pz] = v[q];
     }
     if (!e->d_cpg) {
@@ -872,7 +872,7 @@ static bool setup_tma(ifosb_engine *e, Loop &L) {
     const int nm = (p.nmech == 0 || e->unif_tau) ? 5 : 10;
     const cuuint32_t yb = (cuuint32_t)str_yb(p.nmech);
     const size_t vs = 4 * (size_t)VelSm<VYB>::END;
-    const size_t ss = yb == 4 ? str_box_bytes<4>(nsr, nm) : str_box_bytes<2>(nsr, nm);
+    const size_t ss = yb == 2 ? str_box_bytes<2>(nsr, nm) : str_box_bytes<1>(nsr, nm);
     if (vs > 226 * 1024 || ss > 226 * 1024) return false;
     const cuuint64_t sdims[5] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(p.ny + 5), (cuuint64_t)nslot,
                                  (cuuint64_t)L.nshots};
@@ -932,7 +932,7 @@ static bool dft_step(const ifosb_engine *e, int nt) { return e->nf > 0 && nt % e
 // The velocity ring of a loop that accumulates DFT fields. Called last before the loop,
 // when everything else it needs is allocated: the ring takes at most half of the device
 // memory that is free then, in snapshots of the whole batch, up to MAXRING with the
-// state's own (a 384x256x384, L = 3, nf = 4 shot: 2.70 ms per step with 8), and is
+// state's own (a 384x256x384, L = 3, nf = 4 shot: 2.49 ms per step with 8), and is
 // given back when any later allocation of the engine fails. The time-domain checkpoints
 // of an armed forward read the state's own velocities after every step: no ring.
 static int attach_ring(ifosb_engine *e, Loop &L) {
@@ -1038,8 +1038,8 @@ struct DftRing {
             L.da.v_shot[p] = L.slot_shot[held[p]];
             L.da.trig[p] = L.trig + (size_t)(step[p] - 1) * e->nf * 2;
         }
-        const long long quads = (long long)((e->g.nz + 3) / 4) * e->g.nx * e->g.ny;
-        const dim3 grd((unsigned)((quads + 127) / 128), 3, L.nshots);
+        const long long pairs = (long long)((e->g.nz + 1) / 2) * e->g.nx * e->g.ny;
+        const dim3 grd((unsigned)((pairs + 127) / 128), 3, L.nshots);
         switch (n) {
         case 1: launch_dft_p<1>(L.da, grd, e->stream); break;
         case 2: launch_dft_p<2>(L.da, grd, e->stream); break;

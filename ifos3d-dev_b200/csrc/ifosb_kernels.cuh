@@ -35,7 +35,7 @@ enum { VX = 0, VY, VZ, SYY, SXY, SYZ, SXX, SZZ, SXZ, NEL };
 enum { MD_PI = 0, MD_U, MD_UIPJP, MD_UJPKP, MD_UIPKP, MD_TAUS, MD_TAUP, MD_TSIPJP, MD_TSJPKP, MD_TSIPKP, MD_RIP, MD_RJP, MD_RKP, NMODEL };
 // CPML coefficient rows
 enum { K_X = 0, A_X, B_X, KH_X, AH_X, BH_X, K_Y, A_Y, B_Y, KH_Y, AH_Y, BH_Y, K_Z, A_Z, B_Z, KH_Z, AH_Z, BH_Z,
-       RK_X, RKH_X, RK_Y, RKH_Y, NCPG };  // RK: the correctly rounded reciprocals of K
+       RK_X, RKH_X, RK_Y, RKH_Y, NCPG };  // RK: minus the correctly rounded reciprocals of K
 // The z faces' coefficients per cell (index k-1; K = 1, a = b = 0 inside), so that a
 // thread reads its four cells' as one word. KS, KHS: the stress update's, which takes
 // K_y on the front face (update_s_ssg_CPML_elastic.c:104-108).
@@ -218,37 +218,65 @@ struct DftArgs {
     long long dft_shot;
     int nf;
 };
-// One velocity component (blockIdx.y) of four z-adjacent cells a thread.
+// (float)x as a double: x rounded to nearest even at 24 bits, or at 2^-149 below the
+// normal floats, by adding and subtracting 1.5 * 2^(e+29) (1.5 * 2^-97 at least), whose
+// last place is the float's; a zero keeps x's sign. For |x| < 2^126.
+__device__ __forceinline__ double round24(double x) {
+    const int hi = __double2hiint(x);
+    const double c = __hiloint2double(__viaddmax_s32(hi & 0x7ff00000, 0x01d80000, 0x39e80000), 0);
+    const double r = __dadd_rn(__dadd_rn(x, c), -c);
+    return __hiloint2double((__double2hiint(r) & 0x7fffffff) | (hi & 0x80000000), __double2loint(r));
+}
+// One velocity component (blockIdx.y) of two z-adjacent cells a thread: their velocities
+// of all P steps stay in registers as doubles, eight blocks share an SM, and the next
+// accumulators are on their way while these are updated. The two conversions of every
+// (double)(float) bind the pass to the conversion unit when both cells take them, and
+// round24's integer work to the issue slots when neither does, so one goes each way.
+// 8 steps, nf = 4, 192x160x192: 484 us; 631 (84 % conversion unit) with four
+// cells a thread, 15 warps an SM and conversions only, 736 with round24 only.
 template <int P>
-__global__ void __launch_bounds__(128) k_dft(const __grid_constant__ DftArgs a) {
+__global__ void __launch_bounds__(128, 8) k_dft(const __grid_constant__ DftArgs a) {
+    __shared__ double trig[P][2 * MAXNF];
     const Geo &g = a.g;
-    const int nq = (g.nz + 3) / 4, id = blockIdx.x * blockDim.x + threadIdx.x, row = id / nq;
-    const int j = row / g.nx + 1, i = row % g.nx + 1, k = 4 * (id % nq) + 1, c = blockIdx.y, s = blockIdx.z;
+    const int nl = 2 * a.nf;
+    for (int q = threadIdx.x; q < P * nl; q += 128) trig[q / nl][q % nl] = a.trig[q / nl][q % nl];
+    __syncthreads();
+    const int nq = (g.nz + 1) / 2, id = blockIdx.x * 128 + threadIdx.x, row = id / nq;
+    const int j = row / g.nx + 1, i = row % g.nx + 1, k = 2 * (id % nq) + 1, c = blockIdx.y, s = blockIdx.z;
     if (j > g.ny) return;
     const long long F = g.field, at = (long long)c * F + widx(g, j, i, k);
-    float4 v[P];
+    double v[P][2];
+    float top = 0.f;
 #pragma unroll
-    for (int p = 0; p < P; ++p) v[p] = __ldg(reinterpret_cast<const float4 *>(a.v[p] + (long long)s * a.v_shot[p] + at));
+    for (int p = 0; p < P; ++p) {
+        const float2 x = __ldg(reinterpret_cast<const float2 *>(a.v[p] + (long long)s * a.v_shot[p] + at));
+        v[p][0] = x.x;
+        v[p][1] = x.y;
+        top = fabsf(x.x) < 0x1p100f && fabsf(x.y) < 0x1p100f ? top : INFINITY;  // (NaN too)
+    }
     float *f = a.dft + (long long)s * a.dft_shot + at;
-    const int n = g.nz - k + 1;
-    for (int l = 0; l < 2 * a.nf; ++l, f += 3 * F) {  // cos and sin accumulators in turn
-        const float4 o = *reinterpret_cast<const float4 *>(f);
-        float x[4] = {o.x, o.y, o.z, o.w};
+    float2 o = *reinterpret_cast<const float2 *>(f);
+    for (int l = 0; l < nl; ++l, f += 3 * F) {  // cos and sin accumulators in turn
+        double x0 = o.x, x1 = o.y;
+        const bool fine = top == 0.f && fabsf(o.x) < 0x1p100f;  // far from overflow
+        if (l + 1 < nl) o = *reinterpret_cast<const float2 *>(f + 3 * F);
+        if (fine) {
 #pragma unroll
-        for (int p = 0; p < P; ++p) {
-            const double t = a.trig[p][l];
-            x[0] = (float)((double)x[0] + (double)v[p].x * t);
-            x[1] = (float)((double)x[1] + (double)v[p].y * t);
-            x[2] = (float)((double)x[2] + (double)v[p].z * t);
-            x[3] = (float)((double)x[3] + (double)v[p].w * t);
-        }
-        if (n >= 4) {
-            *reinterpret_cast<float4 *>(f) = make_float4(x[0], x[1], x[2], x[3]);
+            for (int p = 0; p < P; ++p) {
+                const double t = trig[p][l];
+                x0 = round24(__dadd_rn(x0, __dmul_rn(v[p][0], t)));
+                x1 = (double)(float)__dadd_rn(x1, __dmul_rn(v[p][1], t));
+            }
         } else {
 #pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (q < n) f[q] = x[q];
+            for (int p = 0; p < P; ++p) {
+                const double t = trig[p][l];
+                x0 = (double)(float)__dadd_rn(x0, __dmul_rn(v[p][0], t));
+                x1 = (double)(float)__dadd_rn(x1, __dmul_rn(v[p][1], t));
+            }
         }
+        if (k < g.nz) *reinterpret_cast<float2 *>(f) = make_float2((float)x0, (float)x1);
+        else f[0] = (float)x0;
     }
 }
 

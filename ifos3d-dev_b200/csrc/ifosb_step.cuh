@@ -34,13 +34,13 @@ __device__ __forceinline__ Quad quad_of(const Geo &g, int yb) {
 }
 
 // One CPML recursion on a quad: psi' = b psi + a d, d' = d / K + psi'.
-__device__ __forceinline__ F4 pml4(F4 d, F4 old, float *psi, F4 K, F4 RK, F4 A, F4 B, bool fast) {
+__device__ __forceinline__ F4 pml4(F4 d, F4 old, float *psi, F4 K, F4 NRK, F4 A, F4 B, bool fast) {
     const F4 v = B * old + A * d;
     st4(psi, v);
-    return div4(d, K, RK, fast) + v;
+    return div4(d, K, NRK, fast) + v;
 }
-__device__ __forceinline__ F4 pml4(F4 d, F4 old, float *psi, float K, float RK, float A, float B, bool fast) {
-    return pml4(d, old, psi, f4(K), f4(RK), f4(A), f4(B), fast);
+__device__ __forceinline__ F4 pml4(F4 d, F4 old, float *psi, float K, float NRK, float A, float B, bool fast) {
+    return pml4(d, old, psi, f4(K), f4(NRK), f4(A), f4(B), fast);
 }
 
 // Which of the quad's cells lie in a z face of the CPML frame (bit c: cell k+c).
@@ -56,33 +56,41 @@ __device__ __forceinline__ long long szq(const Geo &g, int j, int i, int k) {
     return ((long long)(j - 1) * g.nx + (i - 1)) * g.pzw + (k - 1) + (k > g.fw ? g.zfo : 0);
 }
 
-// The quad's place in the CPML frame and its PML memories, loaded together before the
-// update needs them (the recursions store, and a load after a store waits for it).
+// The quad's place in the CPML frame. Its PML memories are asked for before the update
+// (prefetch into L1, no registers) and read when their axis is done: held in registers
+// from the start, up to nine words a thread, they cost the velocity kernel a fifth of
+// its time at 256^3 (128 registers with spills against 120 without).
 struct Psi {
     int hx, hy, zm;
     float *px, *py, *pz;
-    F4 x[3], y[3], z[3];
 };
-__device__ __forceinline__ void psi_load(Psi &q, const Geo &g, const Slabs &sl, float *ps, int j, int i, int k) {
+__device__ __forceinline__ void prefetch3(const float *p, long long d) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + d));
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 2 * d));
+}
+__device__ __forceinline__ void psi_find(Psi &q, const Geo &g, const Slabs &sl, float *ps, int j, int i, int k) {
     q.hx = face_x(g, i);
     q.hy = face_y(g, j);
     q.zm = face_z_mask(g, k);
     if (q.hx) {
         q.px = ps + sxi(g, j, q.hx, k);
-#pragma unroll
-        for (int n = 0; n < 3; ++n) q.x[n] = ld4(q.px + n * sl.sx);
+        prefetch3(q.px, sl.sx);
     }
     if (q.hy) {
         q.py = ps + 3 * sl.sx + syi(g, q.hy, i, k);
-#pragma unroll
-        for (int n = 0; n < 3; ++n) q.y[n] = ld4(q.py + n * sl.sy);
+        prefetch3(q.py, sl.sy);
     }
     if (q.zm) {
         q.pz = ps + 3 * sl.sx + 3 * sl.sy + szq(g, j, i, k);
-#pragma unroll
-        for (int n = 0; n < 3; ++n) q.z[n] = ld4(q.pz + n * sl.sz);
+        prefetch3(q.pz, sl.sz);
     }
 }
+// An axis's three memories, read together (a load after a recursion's store waits for it).
+struct Psi3 {
+    F4 v[3];
+    __device__ Psi3(const float *p, long long d) : v{ld4(p), ld4(p + d), ld4(p + 2 * d)} {}
+};
 
 // The point forces on a quad's velocities, in list order. pass < 0: the frame's cells
 // before their update; pass 0, 1: after it (an interior cell takes one forward pass,
@@ -165,24 +173,27 @@ __device__ __forceinline__ void vel_quad(const VelArgs &a, const S &m, Psi &q, i
     F4 sxz_x = dx * diff4(b1, S::ld(m.xz), S::ld(m.xz - m.xzI()), b2, S::ld(m.xz + m.xzI()), S::ld(m.xz - 2 * m.xzI()));
     F4 syz_y = dy * diff4(b1, yz0, S::ld(m.yz - m.yzJ()), b2, S::ld(m.yz + m.yzJ()), S::ld(m.yz - 2 * m.yzJ()));
     if (q.hx) {
+        const Psi3 o(q.px, a.sl.sx);
         const int h = q.hx;
         const float K = CPG(cg, K_X, h), RK = CPG(cg, RK_X, h), A = CPG(cg, A_X, h), B = CPG(cg, B_X, h);
-        sxx_x = pml4(sxx_x, q.x[0], q.px, CPG(cg, KH_X, h), CPG(cg, RKH_X, h), CPG(cg, AH_X, h), CPG(cg, BH_X, h), fast);
-        sxy_x = pml4(sxy_x, q.x[1], q.px + a.sl.sx, K, RK, A, B, fast);
-        sxz_x = pml4(sxz_x, q.x[2], q.px + 2 * a.sl.sx, K, RK, A, B, fast);
+        sxx_x = pml4(sxx_x, o.v[0], q.px, CPG(cg, KH_X, h), CPG(cg, RKH_X, h), CPG(cg, AH_X, h), CPG(cg, BH_X, h), fast);
+        sxy_x = pml4(sxy_x, o.v[1], q.px + a.sl.sx, K, RK, A, B, fast);
+        sxz_x = pml4(sxz_x, o.v[2], q.px + 2 * a.sl.sx, K, RK, A, B, fast);
     }
     if (q.hy) {
+        const Psi3 o(q.py, a.sl.sy);
         const int h = q.hy;
         const float K = CPG(cg, K_Y, h), RK = CPG(cg, RK_Y, h), A = CPG(cg, A_Y, h), B = CPG(cg, B_Y, h);
-        sxy_y = pml4(sxy_y, q.y[0], q.py, K, RK, A, B, fast);
-        syy_y = pml4(syy_y, q.y[1], q.py + a.sl.sy, CPG(cg, KH_Y, h), CPG(cg, RKH_Y, h), CPG(cg, AH_Y, h), CPG(cg, BH_Y, h), fast);
-        syz_y = pml4(syz_y, q.y[2], q.py + 2 * a.sl.sy, K, RK, A, B, fast);
+        sxy_y = pml4(sxy_y, o.v[0], q.py, K, RK, A, B, fast);
+        syy_y = pml4(syy_y, o.v[1], q.py + a.sl.sy, CPG(cg, KH_Y, h), CPG(cg, RKH_Y, h), CPG(cg, AH_Y, h), CPG(cg, BH_Y, h), fast);
+        syz_y = pml4(syz_y, o.v[2], q.py + 2 * a.sl.sy, K, RK, A, B, fast);
     }
     if (q.zm) {
+        const Psi3 o(q.pz, a.sl.sz);
         const F4 K = ldg4(cz + Z_K * g.pz), RK = ldg4(cz + Z_RK * g.pz), A = ldg4(cz + Z_A * g.pz), B = ldg4(cz + Z_B * g.pz);
-        sxz_z = sel4(q.zm, pml4(sxz_z, q.z[0], q.pz, K, RK, A, B, fast), sxz_z);
-        syz_z = sel4(q.zm, pml4(syz_z, q.z[1], q.pz + a.sl.sz, K, RK, A, B, fast), syz_z);
-        szz_z = sel4(q.zm, pml4(szz_z, q.z[2], q.pz + 2 * a.sl.sz, ldg4(cz + Z_KH * g.pz), ldg4(cz + Z_RKH * g.pz),
+        sxz_z = sel4(q.zm, pml4(sxz_z, o.v[0], q.pz, K, RK, A, B, fast), sxz_z);
+        syz_z = sel4(q.zm, pml4(syz_z, o.v[1], q.pz + a.sl.sz, K, RK, A, B, fast), syz_z);
+        szz_z = sel4(q.zm, pml4(szz_z, o.v[2], q.pz + 2 * a.sl.sz, ldg4(cz + Z_KH * g.pz), ldg4(cz + Z_RKH * g.pz),
                                 ldg4(cz + Z_AH * g.pz), ldg4(cz + Z_BH * g.pz), fast), szz_z);
     }
     // av_mat's averaged densities (av_mat.c:63-65) from rho and its +1 neighbours; its
@@ -190,9 +201,9 @@ __device__ __forceinline__ void vel_quad(const VelArgs &a, const S &m, Psi &q, i
     const F4 r0 = S::ld(m.rh);
     const F4 rb[3] = {0.5f * (r0 + S::ld(m.rh + m.rhI())), 0.5f * (r0 + S::ld(m.rh + m.rhJ())),
                       0.5f * (r0 + f4(r0.a.y, r0.b.x, r0.b.y, m.rh[4]))};
-    const F4 y[3] = {rcp4(rb[0]), rcp4(rb[1]), rcp4(rb[2])};
+    const F4 ny[3] = {nrcp4(rb[0]), nrcp4(rb[1]), nrcp4(rb[2])};
     F4 d[3] = {sxx_x + sxy_y + sxz_z, syy_y + sxy_x + syz_z, szz_z + sxz_x + syz_y};
-    div4<3>(d, rb, y, fast);
+    div4<3>(d, rb, ny, fast);
     // the frame takes its point forces before the update (update_v() runs first)
     const bool rf = q.hx || q.hy;
     if (p1 > p0) quad_points<BACK>(a, v, p0, p1, j, i, k, nt, rf, q.zm, -1);
@@ -225,7 +236,7 @@ __global__ void __launch_bounds__(QTHR, 4) k_velocity(const __grid_constant__ Ve
     for (int j = Q.j; j <= Q.j1; j += Q.dj) {
         const long long c = widx(g, j, Q.i, Q.k);
         Psi q;
-        psi_load(q, g, a.sl, a.psi + (long long)Q.s * a.psi_shot, j, Q.i, Q.k);
+        psi_find(q, g, a.sl, a.psi + (long long)Q.s * a.psi_shot, j, Q.i, Q.k);
         const float *p = st + c;
         const VelGlobal m{p + SXX * F, p + SYY * F, p + SZZ * F, p + SXY * F, p + SYZ * F, p + SXZ * F, a.rho + c,
                           a.vin + (long long)Q.s * a.vin_shot + c, g.pz, g.plane, F};
@@ -246,7 +257,7 @@ __global__ void __launch_bounds__(QTHR, 4) k_velocity(const __grid_constant__ Ve
 template <bool P2>
 __device__ __forceinline__ F4 dvs(F4 x, float h, float ih, bool fast) {
     if constexpr (P2) return ih * x;
-    else return div4(x, f4(h), f4(ih), fast);
+    else return div4(x, f4(h), f4(-ih), fast);
 }
 // (float)((double)x * s), the reference's promotion of a modulus times (1.0 + L tau)
 __device__ __forceinline__ F4 scale_d(F4 x, double s) {
@@ -301,24 +312,27 @@ __device__ __forceinline__ void str_quad(const StrArgs &a, const S &m, Psi &pq, 
         svyy = vyy;
     }
     if (pq.hx) {
+        const Psi3 o(pq.px, a.sl.sx);
         const int h = pq.hx;
         const float KH = CPG(cg, KH_X, h), RKH = CPG(cg, RKH_X, h), AH = CPG(cg, AH_X, h), BH = CPG(cg, BH_X, h);
-        vxx = pml4(vxx, pq.x[0], pq.px, CPG(cg, K_X, h), CPG(cg, RK_X, h), CPG(cg, A_X, h), CPG(cg, B_X, h), fast);
-        vyx = pml4(vyx, pq.x[1], pq.px + a.sl.sx, KH, RKH, AH, BH, fast);
-        vzx = pml4(vzx, pq.x[2], pq.px + 2 * a.sl.sx, KH, RKH, AH, BH, fast);
+        vxx = pml4(vxx, o.v[0], pq.px, CPG(cg, K_X, h), CPG(cg, RK_X, h), CPG(cg, A_X, h), CPG(cg, B_X, h), fast);
+        vyx = pml4(vyx, o.v[1], pq.px + a.sl.sx, KH, RKH, AH, BH, fast);
+        vzx = pml4(vzx, o.v[2], pq.px + 2 * a.sl.sx, KH, RKH, AH, BH, fast);
     }
     if (pq.hy) {
+        const Psi3 o(pq.py, a.sl.sy);
         const int h = pq.hy;
         const float KH = CPG(cg, KH_Y, h), RKH = CPG(cg, RKH_Y, h), AH = CPG(cg, AH_Y, h), BH = CPG(cg, BH_Y, h);
-        vxy = pml4(vxy, pq.y[0], pq.py, KH, RKH, AH, BH, fast);
-        vyy = pml4(vyy, pq.y[1], pq.py + a.sl.sy, CPG(cg, K_Y, h), CPG(cg, RK_Y, h), CPG(cg, A_Y, h), CPG(cg, B_Y, h), fast);
-        vzy = pml4(vzy, pq.y[2], pq.py + 2 * a.sl.sy, KH, RKH, AH, BH, fast);
+        vxy = pml4(vxy, o.v[0], pq.py, KH, RKH, AH, BH, fast);
+        vyy = pml4(vyy, o.v[1], pq.py + a.sl.sy, CPG(cg, K_Y, h), CPG(cg, RK_Y, h), CPG(cg, A_Y, h), CPG(cg, B_Y, h), fast);
+        vzy = pml4(vzy, o.v[2], pq.py + 2 * a.sl.sy, KH, RKH, AH, BH, fast);
     }
     if (pq.zm) {
+        const Psi3 o(pq.pz, a.sl.sz);
         const F4 KH = ldg4(cz + Z_KHS * g.pz), RKH = ldg4(cz + Z_RKHS * g.pz), AH = ldg4(cz + Z_AH * g.pz), BH = ldg4(cz + Z_BH * g.pz);
-        vxz = sel4(pq.zm, pml4(vxz, pq.z[0], pq.pz, KH, RKH, AH, BH, fast), vxz);
-        vyz = sel4(pq.zm, pml4(vyz, pq.z[1], pq.pz + a.sl.sz, KH, RKH, AH, BH, fast), vyz);
-        vzz = sel4(pq.zm, pml4(vzz, pq.z[2], pq.pz + 2 * a.sl.sz, ldg4(cz + Z_KS * g.pz), ldg4(cz + Z_RKS * g.pz),
+        vxz = sel4(pq.zm, pml4(vxz, o.v[0], pq.pz, KH, RKH, AH, BH, fast), vxz);
+        vyz = sel4(pq.zm, pml4(vyz, o.v[1], pq.pz + a.sl.sz, KH, RKH, AH, BH, fast), vyz);
+        vzz = sel4(pq.zm, pml4(vzz, o.v[2], pq.pz + 2 * a.sl.sz, ldg4(cz + Z_KS * g.pz), ldg4(cz + Z_RKS * g.pz),
                                ldg4(cz + Z_A * g.pz), ldg4(cz + Z_B * g.pz), fast), vzz);
     }
     const F4 vxyyx = vxy + vyx, vyzzy = vyz + vzy, vxzzx = vxz + vzx;
@@ -514,7 +528,7 @@ __global__ void __launch_bounds__(QTHR, 4) k_stress(const __grid_constant__ StrA
     for (int j = Q.j; j <= Q.j1; j += Q.dj) {
         const long long c = widx(g, j, Q.i, Q.k);
         Psi q;
-        psi_load(q, g, a.sl, a.psi + (long long)Q.s * a.psi_shot + 3 * (a.sl.sx + a.sl.sy + a.sl.sz), j, Q.i, Q.k);
+        psi_find(q, g, a.sl, a.psi + (long long)Q.s * a.psi_shot + 3 * (a.sl.sx + a.sl.sy + a.sl.sz), j, Q.i, Q.k);
         const float *p = a.st + (long long)Q.s * a.st_shot + c;
         const float *v = a.v + (long long)Q.s * a.v_shot + c;
         const StrGlobal m{v + VX * F, v + VY * F, v + VZ * F, p + SYY * F, a.md + c, g.pz, g.plane, F};
