@@ -106,6 +106,8 @@ struct StrBox {
 constexpr int VYB = 2;
 __host__ __device__ constexpr int str_yb(int nmech) { return nmech == 0 ? 2 : 1; }
 
+constexpr unsigned ONE_WAVE = 4 * 148;  // CTAs resident at once
+
 // This thread's cells in a CTA's box, and the chunk's planes.
 struct BoxAt {
     int k0, i0, s, yc, j0, j1, zq, x, y, k, i;
@@ -138,6 +140,7 @@ __device__ __forceinline__ void box_loop(uint64_t *full, int *err, WaitCtl w, in
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
+    pdl_wait();
     const int flag = *(volatile const int *)err;
     const int n = (b.j1 - b.j0 + YB) / YB;
     for (int it = 0; it < n; ++it) {
@@ -156,6 +159,9 @@ __device__ __forceinline__ void box_loop(uint64_t *full, int *err, WaitCtl w, in
             if (threadIdx.x == 0 && issue) mbar_wait(full, it & 1, w.limit_ns);
         }
         ok = ok && flag == 0;
+        // the next kernel's CTAs may move in once the boxes of the last wave have landed; a
+        // grid of one wave keeps its SMs to itself until it ends
+        if (it == 0 && gridDim.x * gridDim.y * gridDim.z > ONE_WAVE) pdl_release();
         if (active && ok) update(j);
         // every thread has read the box before the next one lands in it
         if (it + 1 < n && !__syncthreads_and(ok)) return;

@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "ifosb_tma.cuh"
+
 namespace ifosb {
 
 constexpr int MAXFW = 64;
@@ -239,8 +241,10 @@ __global__ void __launch_bounds__(128, 8) k_dft(const __grid_constant__ DftArgs 
     __shared__ double trig[P][2 * MAXNF];
     const Geo &g = a.g;
     const int nl = 2 * a.nf;
+    pdl_release();
     for (int q = threadIdx.x; q < P * nl; q += 128) trig[q / nl][q % nl] = a.trig[q / nl][q % nl];
     __syncthreads();
+    pdl_wait();
     const int nq = (g.nz + 1) / 2, id = blockIdx.x * 128 + threadIdx.x, row = id / nq;
     const int j = row / g.nx + 1, i = row % g.nx + 1, k = 2 * (id % nq) + 1, c = blockIdx.y, s = blockIdx.z;
     if (j > g.ny) return;
@@ -281,29 +285,6 @@ __global__ void __launch_bounds__(128, 8) k_dft(const __grid_constant__ DftArgs 
 }
 
 // ---------------------------------------------------------------------------
-// gradient_F (gradient_F.c:62-139): for every shot of the batch (in order) and
-// every frequency, the 4th-order derivatives of the forward and backward DFT
-// fields are multiplied into the vp, vs, rho gradients. grad is compact
-// [3][NY][NX][NZ]; grad64 accumulates the same contributions in FP64.
-struct GradArgs {
-    Geo g;
-    const float *dftf, *dftb;  // [shot][nf][6][field]
-    long long dft_shot;
-    int nshots, nf;
-    const float *md;           // model: rho is taken from the ghosted rho slot
-    const float *rho;          // rho in field layout
-    float fdummy[MAXNF];       // 1/(4 pi^2 f^2) in float as gradient_F.c:70-72
-    float b1, b2, rdx, rdy, rdz;
-    float ihx, ihy, ihz;       // 1/DX, 1/DY, 1/DZ (exact for power-of-two spacings)
-    float *grad;
-    double *grad64;
-    // viscoelastic only: gradients with respect to taup and taus ([2][NY][NX][NZ],
-    // FP64), with Phi(omega_l) = sum_m s tau_m / (1 + s tau_m), s = -i omega_l,
-    // tau_m = DT / eta_m (the memory-variable relaxation of update_s_ssg.c:108-122)
-    double *gradq;
-    double rphi[MAXNF], iphi[MAXNF];
-};
-
 // x / h with the division operator's bits: for a power-of-two spacing the exact
 // reciprocal (x * (1/h) == x / h for h = 2^k), else div_rn (no slow path for the
 // zero dividends of a field the wave has not reached)
@@ -312,7 +293,7 @@ __device__ __forceinline__ float dvh(float x, float h, float ih) {
     return P2 ? __fmul_rn(x, ih) : div_rn(x, h);
 }
 
-// d: a float[9] or a column of shared memory (SCol); DX.. the spacings, IX.. their
+// d: a float[9]; DX.. the spacings, IX.. their
 // reciprocals (used with P2)
 template <bool P2, class D>
 __device__ __forceinline__ void dft_derivs(const float *X, const float *Y, const float *Z, long long c, long long dI,
@@ -333,125 +314,6 @@ __device__ __forceinline__ void dft_derivs(const float *X, const float *Y, const
 __device__ __forceinline__ const float *opaque(const float *p) {
     asm volatile("" : "+l"(p));
     return p;
-}
-
-// Nine values of one thread in shared memory, stride one block: the kernel keeps
-// its 36 derivatives there instead of in registers.
-struct SCol {
-    float *p;
-    __device__ __forceinline__ float &operator[](int q) const { return p[q * (BX * BY)]; }
-};
-
-// Q: also the viscoelastic taup / taus gradient (a.gradq). Two instances, so the
-// elastic one keeps the registers of gradient_F's terms alone. The kernel is
-// latency-bound on its 156 loads per cell, shot and frequency. Left to itself the
-// compiler hoisted all of them (and their 64-bit addresses) and used 243-254
-// registers: one block per SM, or spills that went to DRAM at lower caps. With
-// the derivatives in shared memory and each stencil set's pointers opaque, four
-// blocks per SM fit in 62-64 registers: 5.7 ms instead of 18.4 ms for 4 shots x
-// 4 frequencies at 128^3, L=3 (0.66 instead of 2.0 ms elastic, nf=2), same bits.
-#ifndef IFOSB_GRAD_MINB
-#define IFOSB_GRAD_MINB 4
-#endif
-template <bool Q, bool P2>
-__global__ void __launch_bounds__(BX *BY, IFOSB_GRAD_MINB) k_gradient(GradArgs a) {
-    __shared__ float sdv[4 * 9 * BX * BY];
-    const Geo &g = a.g;
-    const int k = blockIdx.x * BX + threadIdx.x + 1;
-    const int i = blockIdx.y * BY + threadIdx.y + 1;
-    const int tid = threadIdx.y * BX + threadIdx.x;
-    const SCol fv{sdv + tid}, bv{sdv + 9 * BX * BY + tid}, fi{sdv + 18 * BX * BY + tid}, bi{sdv + 27 * BX * BY + tid};
-    const int yc = blockIdx.z;
-    if (k > g.nz || i > g.nx) return;
-    const int j0 = yc * g.cy + 1;
-    const int j1 = min(j0 + g.cy - 1, g.ny);
-    const long long F = g.field, dI = g.pz, dJ = g.plane;
-    const long long n = (long long)g.nx * g.ny * g.nz;
-    for (int j = j0; j <= j1; ++j) {
-        const long long c = widx(g, j, i, k);
-        const long long m = ((long long)(j - 1) * g.nx + (i - 1)) * g.nz + (k - 1);
-        float g1 = a.grad[m], g2 = a.grad[n + m], g3 = a.grad[2 * n + m];
-        double h1 = a.grad64[m], h2 = a.grad64[n + m], h3 = a.grad64[2 * n + m];
-        double qp = 0.0, qs = 0.0;
-        if (Q) {
-            qp = a.gradq[m];
-            qs = a.gradq[n + m];
-        }
-        const float r = a.rho[c], pp = a.md[MD_PI * F + c], uu = a.md[MD_U * F + c];
-        const double sqp = sqrt((double)(r * pp)), squ = sqrt((double)(r * uu));
-        for (int s = 0; s < a.nshots; ++s) {
-            for (int l = 0; l < a.nf; ++l) {
-                const float *Fb = a.dftf + (long long)s * a.dft_shot + (long long)l * 6 * F;
-                const float *Bb = a.dftb + (long long)s * a.dft_shot + (long long)l * 6 * F;
-                // One stencil set at a time: each set's field pointers pass through an
-                // empty asm, so the compiler can neither hoist the 36 addresses of all
-                // sets out of the loops nor issue the next set's loads early; the
-                // 144 loads then need few registers (no spills to local memory).
-                const float *Fc = Fb + c, *Bc = Bb + c;
-                const float *p0 = opaque(Fc), *p1 = opaque(Fc + F), *p2 = opaque(Fc + 2 * F);
-                dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, fv);
-                p0 = opaque(Bc); p1 = opaque(Bc + F); p2 = opaque(Bc + 2 * F);
-                dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, bv);
-                p0 = opaque(Fc + 3 * F); p1 = opaque(Fc + 4 * F); p2 = opaque(Fc + 5 * F);
-                dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, fi);
-                p0 = opaque(Bc + 3 * F); p1 = opaque(Bc + 4 * F); p2 = opaque(Bc + 5 * F);
-                dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, bi);
-                const float fdummy = a.fdummy[l];
-                float gradlam = (fv[0] + fv[4] + fv[8]) * (bv[0] + bv[4] + bv[8]) + (fi[0] + fi[4] + fi[8]) * (bi[0] + bi[4] + bi[8]);
-                gradlam = -gradlam * fdummy;
-                float gradmu = 2.0f * fv[0] * bv[0] + 2.0f * fv[4] * bv[4] + 2.0f * fv[8] * bv[8] + 2.0f * fi[0] * bi[0] +
-                               2.0f * fi[4] * bi[4] + 2.0f * fi[8] * bi[8] + (fv[1] + fv[3]) * (bv[1] + bv[3]) +
-                               (fi[1] + fi[3]) * (bi[1] + bi[3]) + (fv[2] + fv[6]) * (bv[2] + bv[6]) +
-                               (fi[2] + fi[6]) * (bi[2] + bi[6]) + (fv[5] + fv[7]) * (bv[5] + bv[7]) +
-                               (fi[5] + fi[7]) * (bi[5] + bi[7]);
-                gradmu = -gradmu * fdummy;
-                const float gradrho = (Fb[c] * Bb[c] + Fb[F + c] * Bb[F + c] + Fb[2 * F + c] * Bb[2 * F + c]) +
-                                      (Fb[3 * F + c] * Bb[3 * F + c] + Fb[4 * F + c] * Bb[4 * F + c] + Fb[5 * F + c] * Bb[5 * F + c]);
-                const double c1 = sqp * 2.0 * (double)gradlam;
-                const double c2 = -4.0 * squ * (double)gradlam + 2.0 * squ * (double)gradmu;
-                const float c3 = gradrho + uu / r * gradmu + (pp - 2.0f * uu) / r * gradlam;
-                g1 = (float)((double)g1 + c1);
-                g2 = (float)((double)g2 + c2);
-                g3 = g3 + c3;
-                h1 += c1;
-                h2 += c2;
-                h3 += (double)c3;
-                if (Q) {
-                    // complex correlations C = F conj(B) of the lambda and mu terms with
-                    // gradient_F's factor -fdummy: its gradlam / gradmu are their real
-                    // parts. A modulus M(1 + tau Phi) perturbed in tau moves the misfit
-                    // by Re[M Phi C] (lambda part for taup; mu - 2 lambda for taus).
-                    const double fd = -(double)fdummy;
-                    const double dfr = (double)fv[0] + fv[4] + fv[8], dfi = (double)fi[0] + fi[4] + fi[8];
-                    const double dbr = (double)bv[0] + bv[4] + bv[8], dbi = (double)bi[0] + bi[4] + bi[8];
-                    const double rl = fd * (dfr * dbr + dfi * dbi), il = fd * (dfi * dbr - dfr * dbi);
-                    double rm = 0.0, im = 0.0;
-                    for (int q = 0; q < 9; q += 4) {  // xx, yy, zz
-                        rm += 2.0 * ((double)fv[q] * bv[q] + (double)fi[q] * bi[q]);
-                        im += 2.0 * ((double)fi[q] * bv[q] - (double)fv[q] * bi[q]);
-                    }
-                    const int pr[3][2] = {{1, 3}, {2, 6}, {5, 7}};  // xy, xz, yz
-                    for (int q = 0; q < 3; ++q) {
-                        const double fr = (double)fv[pr[q][0]] + fv[pr[q][1]], fim = (double)fi[pr[q][0]] + fi[pr[q][1]];
-                        const double br = (double)bv[pr[q][0]] + bv[pr[q][1]], bim = (double)bi[pr[q][0]] + bi[pr[q][1]];
-                        rm += fr * br + fim * bim;
-                        im += fim * br - fr * bim;
-                    }
-                    rm *= fd;
-                    im *= fd;
-                    const double ph = a.rphi[l], qh = a.iphi[l];
-                    qp += (double)pp * (ph * rl - qh * il);
-                    qs += (double)uu * (ph * (rm - 2.0 * rl) - qh * (im - 2.0 * il));
-                }
-            }
-        }
-        a.grad[m] = g1; a.grad[n + m] = g2; a.grad[2 * n + m] = g3;
-        a.grad64[m] = h1; a.grad64[n + m] = h2; a.grad64[2 * n + m] = h3;
-        if (Q) {
-            a.gradq[m] = qp;
-            a.gradq[n + m] = qs;
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -553,105 +415,6 @@ __global__ void k_td_integrate(float *u, const float *st, long long st_shot, lon
             SV[q] = v;
             SU[q] = x;
         }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// hess_F (hess_F.c:67-155): the diagonal approximate Hessian from the forward DFT
-// fields of every shot of the batch (in order) and the DFT fields of the
-// receivers' Green's functions (wavefields of a y-force at each receiver), for
-// every frequency. hess is compact [3][NY][NX][NZ] FP32, accumulated in the
-// reference's order: shots, then receivers, then frequencies.
-struct HessArgs {
-    Geo g;
-    const float *dftf;         // [shot][nf][6][field]
-    long long dft_shot;
-    const float *green;        // [receiver][nf][6][field] (same per-entry stride)
-    int nshots, nrec, nf;
-    const float *md;           // model: pi, u slots
-    const float *rho;          // rho in field layout
-    float fdummy[MAXNF];       // 1/(2 pi f) in float as hess_F.c:72-74
-    float b1, b2, rdx, rdy, rdz;
-    float ihx, ihy, ihz;       // 1/DX, 1/DY, 1/DZ (exact for power-of-two spacings)
-    float *hess;
-};
-
-// With the derivatives in shared memory and opaque stencil pointers (as in
-// k_gradient), four blocks per SM fit in 62 registers without spills: 35.5 ms
-// for 2 shots x 25 receivers x 2 frequencies at 128^3, against 98 ms at one
-// block (236 registers) and 62 ms at two (128, with spills); same bits.
-#ifndef IFOSB_HESS_MINB
-#define IFOSB_HESS_MINB 4
-#endif
-template <bool P2>
-__global__ void __launch_bounds__(BX *BY, IFOSB_HESS_MINB) k_hessian(HessArgs a) {
-    __shared__ float sdv[4 * 9 * BX * BY];
-    const Geo &g = a.g;
-    const int k = blockIdx.x * BX + threadIdx.x + 1;
-    const int i = blockIdx.y * BY + threadIdx.y + 1;
-    const int tid = threadIdx.y * BX + threadIdx.x;
-    const SCol fv{sdv + tid}, bv{sdv + 9 * BX * BY + tid}, fi{sdv + 18 * BX * BY + tid}, bi{sdv + 27 * BX * BY + tid};
-    const int yc = blockIdx.z;
-    if (k > g.nz || i > g.nx) return;
-    const int j0 = yc * g.cy + 1;
-    const int j1 = min(j0 + g.cy - 1, g.ny);
-    const long long F = g.field, dI = g.pz, dJ = g.plane;
-    const long long n = (long long)g.nx * g.ny * g.nz;
-    for (int j = j0; j <= j1; ++j) {
-        const long long c = widx(g, j, i, k);
-        const long long m = ((long long)(j - 1) * g.nx + (i - 1)) * g.nz + (k - 1);
-        float h1 = a.hess[m], h2 = a.hess[n + m], h3 = a.hess[2 * n + m];
-        const float r = a.rho[c], pp = a.md[MD_PI * F + c], uu = a.md[MD_U * F + c];
-        for (int s = 0; s < a.nshots; ++s) {
-            for (int q = 0; q < a.nrec; ++q) {
-                for (int l = 0; l < a.nf; ++l) {
-                    const float *Fb = a.dftf + (long long)s * a.dft_shot + (long long)l * 6 * F;
-                    const float *Bb = a.green + (long long)q * a.dft_shot + (long long)l * 6 * F;
-                    // one stencil set at a time, as in k_gradient
-                    const float *Fc = Fb + c, *Bc = Bb + c;
-                    const float *p0 = opaque(Fc), *p1 = opaque(Fc + F), *p2 = opaque(Fc + 2 * F);
-                    dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, fv);
-                    p0 = opaque(Bc); p1 = opaque(Bc + F); p2 = opaque(Bc + 2 * F);
-                    dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, bv);
-                    p0 = opaque(Fc + 3 * F); p1 = opaque(Fc + 4 * F); p2 = opaque(Fc + 5 * F);
-                    dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, fi);
-                    p0 = opaque(Bc + 3 * F); p1 = opaque(Bc + 4 * F); p2 = opaque(Bc + 5 * F);
-                    dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, bi);
-                    const float fd = a.fdummy[l];
-                    const float fdiv = fv[0] + fv[4] + fv[8], fidiv = fi[0] + fi[4] + fi[8];
-                    const float bdiv = bv[0] + bv[4] + bv[8], bidiv = bi[0] + bi[4] + bi[8];
-                    float relam = fidiv * bdiv + fdiv * bidiv;
-                    relam = fd * relam;
-                    float imlam = fidiv * bidiv - fdiv * bdiv;
-                    imlam = fd * imlam;
-                    float remu = 2.0f * fi[0] * bv[0] + 2.0f * fi[4] * bv[4] + 2.0f * fi[8] * bv[8] +
-                                 2.0f * fv[0] * bi[0] + 2.0f * fv[4] * bi[4] + 2.0f * fv[8] * bi[8] +
-                                 (fi[1] + fi[3]) * (bv[1] + bv[3]) + (fv[1] + fv[3]) * (bi[1] + bi[3]) +
-                                 (fi[2] + fi[6]) * (bv[2] + bv[6]) + (fv[2] + fv[6]) * (bi[2] + bi[6]) +
-                                 (fi[5] + fi[7]) * (bv[5] + bv[7]) + (fv[5] + fv[7]) * (bi[5] + bi[7]);
-                    remu = fd * remu;
-                    float immu = 2.0f * fi[0] * bi[0] + 2.0f * fi[4] * bi[4] + 2.0f * fi[8] * bi[8] -
-                                 2.0f * fv[0] * bv[0] - 2.0f * fv[4] * bv[4] - 2.0f * fv[8] * bv[8] +
-                                 (fi[1] + fi[3]) * (bi[1] + bi[3]) - (fv[1] + fv[3]) * (bv[1] + bv[3]) +
-                                 (fi[2] + fi[6]) * (bi[2] + bi[6]) - (fv[2] + fv[6]) * (bv[2] + bv[6]) +
-                                 (fi[5] + fi[7]) * (bi[5] + bi[7]) - (fv[5] + fv[7]) * (bv[5] + bv[7]);
-                    immu = fd * immu;
-                    const float rerho = (Fb[c] * Bb[c] + Fb[F + c] * Bb[F + c] + Fb[2 * F + c] * Bb[2 * F + c]) -
-                                        (Fb[3 * F + c] * Bb[3 * F + c] + Fb[4 * F + c] * Bb[4 * F + c] +
-                                         Fb[5 * F + c] * Bb[5 * F + c]);
-                    const float imrho = (Fb[c] * Bb[3 * F + c] + Fb[F + c] * Bb[4 * F + c] + Fb[2 * F + c] * Bb[5 * F + c]) +
-                                        (Fb[3 * F + c] * Bb[c] + Fb[4 * F + c] * Bb[F + c] + Fb[5 * F + c] * Bb[2 * F + c]);
-                    const float revs = -2.0f * relam + remu;
-                    const float imvs = -2.0f * imlam + immu;
-                    const float rerho1 = rerho + relam * (pp - 2.0f * uu) / r + remu * uu / r;
-                    const float imrho1 = imrho + imlam * (pp - 2.0f * uu) / r + immu * uu / r;
-                    h1 += (relam * relam + imlam * imlam) * r * pp * 4.0f;
-                    h2 += (revs * revs + imvs * imvs) * 4.0f * r * uu;
-                    h3 += rerho1 * rerho1 + imrho1 * imrho1;
-                }
-            }
-        }
-        a.hess[m] = h1; a.hess[n + m] = h2; a.hess[2 * n + m] = h3;
     }
 }
 

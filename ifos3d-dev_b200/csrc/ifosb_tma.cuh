@@ -3,7 +3,7 @@
 #pragma once
 #include <cuda.h>
 
-#include "ifosb_kernels.cuh"
+#include <stdint.h>
 
 namespace ifosb {
 
@@ -99,6 +99,13 @@ __device__ __forceinline__ void tma_prefetch4(const CUtensorMap *m, int c0, int 
 __device__ __forceinline__ int zc(int k) { return k + 7; }
 __device__ __forceinline__ int xc(int i) { return i + 1; }
 __device__ __forceinline__ int yc_(int j) { return j + 2; }
+
+// Programmatic dependent launch: a kernel of the time loop may let its successor's CTAs
+// take their places before it ends (all of its own have called pdl_release or ended),
+// and waits itself, before it touches anything the loop writes, until its predecessor
+// has finished and its writes are visible. Without the launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Failure-path test knobs: the mbarrier wait limit, and the box of a chunk from which
 // on a CTA issues no more loads (-1 = never); the waits for boxes never issued run out.
