@@ -1761,7 +1761,7 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
 // gradient comes out with respect to the raw model ifosb_set_model received,
 // interior cells, [5][NY*NX*NZ]: rho, pi, u, taus, taup (the last two zero for
 // L = 0).
-static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double *misfit) {
+static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *gmod, double *misfit) {
     if (!e || !misfit || interval < 1) return IFOSB_EARG;
     const ifosb_params &p = e->p;
     if (!e->fwd_ok || !e->res_ok) return fail(e, IFOSB_ESTATE, "the exact VJP needs a forward batch and its residual");
@@ -1790,7 +1790,12 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double 
         CU(cudaMemsetAsync(blk, 0, total * sizeof(double), e->stream));
         const size_t ng = (size_t)(p.nx + 2) * (p.ny + 2) * (p.nz + 2);
         const float *raw = e->d_mstage;  // rho, pi, u, taus, taup as ifosb_set_model received them (ghosted)
-        const dim3 blk3(128), grd3((p.nz + 127) / 128, p.nx, p.ny);
+        decltype(&k64_str<0>) const strs[MAXMECH + 1] = {k64_str<0>, k64_str<1>, k64_str<2>, k64_str<3>, k64_str<4>};
+        decltype(&k64_str_T<0>) const strTs[MAXMECH + 1] = {k64_str_T<0>, k64_str_T<1>, k64_str_T<2>, k64_str_T<3>, k64_str_T<4>};
+        const auto str64 = strs[L];
+        const auto str64_T = strTs[L];
+        const unsigned bz = (p.nz + V64Z - 1) / V64Z, bx = (p.nx + V64X - 1) / V64X;
+        const dim3 blk3(V64Z, V64X), grd3(bz, bx, p.ny);
         k64_model<<<grd3, blk3, 0, e->stream>>>(g, raw, raw + ng, raw + 2 * ng, L ? raw + 3 * ng : nullptr,
                                                  L ? raw + 4 * ng : nullptr, md);
         Vjp64 a{};
@@ -1846,7 +1851,7 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double 
             auto step = [&](double *st, int nt) {
                 double *ps = st + (size_t)NELV * F;
                 k64_vel<<<grd3, blk3, 0, e->stream>>>(a, st, ps);
-                k64_str<<<grd3, blk3, 0, e->stream>>>(a, st, ps, nt);
+                str64<<<grd3, blk3, 0, e->stream>>>(a, st, ps, nt);
             };
             // 1. the forward from rest, checkpoints after steps 0, K, 2K, ..., the traces
             double *w = seg;
@@ -1890,8 +1895,8 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double 
             CU(cudaMemsetAsync(lam, 0, SZ * sizeof(double), e->stream));
             CU(cudaMemsetAsync(ld, 0, 18 * (size_t)F * sizeof(double), e->stream));
             double *lps = lam + (size_t)NELV * F;
-            const dim3 grdg((p.nz + 127) / 128, p.nx, p.ny + (g.free_surf ? 2 : 0));
-            const dim3 grds((p.nz + 127) / 128, p.nx);
+            const dim3 grdg(bz, bx, p.ny + (g.free_surf ? 2 : 0));
+            const dim3 grds(bz, bx);
             for (int q = nseg - 1; q >= 0; --q) {
                 const int a0 = q * K + 1, a1 = std::min((q + 1) * K, NT);
                 CU(cudaMemcpyAsync(seg, ck + (size_t)q * SZ, SZ * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
@@ -1904,7 +1909,7 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double 
                     const double *cur = seg + (size_t)(nt - a0 + 1) * SZ, *prev = cur - SZ;
                     k64_inject<<<(ntr + 127) / 128, 128, 0, e->stream>>>(g, lam, drec, ntr, ns, nt - 1, asrc);
                     if (g.free_surf) k64_mirror_T<<<grds, blk3, 0, e->stream>>>(g, lam);
-                    k64_str_T<<<grd3, blk3, 0, e->stream>>>(a, lam, lps, ld, cur, prev + (size_t)NELV * F, gr);
+                    str64_T<<<grd3, blk3, 0, e->stream>>>(a, lam, lps, ld, cur, prev + (size_t)NELV * F, gr);
                     k64_str_T_gather<<<grd3, blk3, 0, e->stream>>>(a, lam, ld);
                     k64_vel_T<<<grd3, blk3, 0, e->stream>>>(a, lam, lps, ls, cur, prev, gr);
                     k64_vel_T_gather<<<grdg, blk3, 0, e->stream>>>(a, lam, ls, g.free_surf ? -1 : 1);
@@ -1913,63 +1918,14 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double 
             }
         }
         if (!gmod) return IFOSB_OK;
-        // 4. the averaged moduli's gradients onto the raw model (av_mat.c:45-69 and
-        //    matcopy's periodic ghost layers)
-        std::vector<double> gh((size_t)N64 * n);
-        std::vector<float> rawh(3 * ng);
-        CU(cudaMemcpyAsync(gh.data(), gq, gh.size() * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-        CU(cudaMemcpyAsync(rawh.data(), raw, rawh.size() * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+        // 4. the coefficients' gradients onto the raw model, in the states' place
+        double *fold = ck;
+        const int nq = chain ? 3 : 5;
+        k64_fold<<<grd3, blk3, 0, e->stream>>>(g, gr, md, raw, L, chain, fold);
+        int r;
+        if ((r = check_launch(e, "exact VJP gradient"))) return r;
+        CU(cudaMemcpyAsync(gmod, fold, (size_t)nq * n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
         CU(cudaStreamSynchronize(e->stream));
-        const int NX = p.nx, NY = p.ny, NZ = p.nz, GX = NX + 2, GZ = NZ + 2;
-        auto G = [&](int j, int i, int k) { return ((size_t)j * GX + i) * GZ + k; };
-        const float *u = rawh.data() + 2 * ng;
-        // ghosted accumulators in the order of the output: rho, pi, u, taus, taup
-        std::vector<double> acc(5 * ng, 0.0);
-        double *dr = acc.data(), *dp = dr + ng, *du = dp + ng, *dts = du + ng, *dtp = dts + ng;
-        auto harm = [&](double gval, int j0, int i0, int k0, int j1, int i1, int k1, int j2, int i2, int k2, int j3,
-                        int i3, int k3) {
-            const size_t c[4] = {G(j0, i0, k0), G(j1, i1, k1), G(j2, i2, k2), G(j3, i3, k3)};
-            double s = 0.0;
-            for (size_t q : c) s += 1.0 / (double)u[q];
-            const double avg = 4.0 / s;
-            for (size_t q : c) du[q] += gval * avg * avg / (4.0 * (double)u[q] * (double)u[q]);
-        };
-        auto quarter = [&](double gval, int j0, int i0, int k0, int j1, int i1, int k1, int j2, int i2, int k2, int j3,
-                           int i3, int k3) {
-            dts[G(j0, i0, k0)] += 0.25 * gval; dts[G(j1, i1, k1)] += 0.25 * gval;
-            dts[G(j2, i2, k2)] += 0.25 * gval; dts[G(j3, i3, k3)] += 0.25 * gval;
-        };
-        for (int j = 1; j <= NY; ++j)
-            for (int i = 1; i <= NX; ++i)
-                for (int k = 1; k <= NZ; ++k) {
-                    const size_t m = ((size_t)(j - 1) * NX + (i - 1)) * NZ + (k - 1), c = G(j, i, k);
-                    auto gv = [&](int q) { return gh[(size_t)q * n + m]; };
-                    dp[c] += gv(M64_PI);
-                    du[c] += gv(M64_U);
-                    dr[c] += 0.5 * gv(M64_RIP); dr[G(j, i + 1, k)] += 0.5 * gv(M64_RIP);
-                    dr[c] += 0.5 * gv(M64_RJP); dr[G(j + 1, i, k)] += 0.5 * gv(M64_RJP);
-                    dr[c] += 0.5 * gv(M64_RKP); dr[G(j, i, k + 1)] += 0.5 * gv(M64_RKP);
-                    harm(gv(M64_UIPJP), j, i, k, j, i + 1, k, j + 1, i + 1, k, j + 1, i, k);
-                    harm(gv(M64_UJPKP), j, i, k, j, i, k + 1, j + 1, i, k + 1, j + 1, i, k);
-                    harm(gv(M64_UIPKP), j, i, k, j, i, k + 1, j, i + 1, k + 1, j, i + 1, k);
-                    if (L) {  // tausipjp ... are plain means of four cells (av_mat.c:57-59)
-                        dts[c] += gv(M64_TAUS);
-                        dtp[c] += gv(M64_TAUP);
-                        quarter(gv(M64_TSIPJP), j, i, k, j, i + 1, k, j + 1, i + 1, k, j + 1, i, k);
-                        quarter(gv(M64_TSJPKP), j, i, k, j + 1, i, k, j + 1, i, k + 1, j, i, k + 1);
-                        quarter(gv(M64_TSIPKP), j, i, k, j, i + 1, k, j, i + 1, k + 1, j, i, k + 1);
-                    }
-                }
-        // fold the ghost layers (matcopy on one rank: index 0 = N, N + 1 = 1)
-        auto wrapi = [](int x, int N) { return x == 0 ? N : (x == N + 1 ? 1 : x); };
-        std::fill(gmod, gmod + 5 * n, 0.0);
-        for (int j = 0; j <= NY + 1; ++j)
-            for (int i = 0; i <= NX + 1; ++i)
-                for (int k = 0; k <= NZ + 1; ++k) {
-                    const size_t c = G(j, i, k);
-                    const size_t m = ((size_t)(wrapi(j, NY) - 1) * NX + (wrapi(i, NX) - 1)) * NZ + (wrapi(k, NZ) - 1);
-                    for (int q = 0; q < 5; ++q) gmod[(size_t)q * n + m] += acc[(size_t)q * ng + c];
-                }
         return IFOSB_OK;
     };
     rc = run();
@@ -1981,36 +1937,16 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, double *gmod, double 
 }
 
 extern "C" int ifosb_vjp_exact_moduli(ifosb_engine *e, int interval, double *grad, double *misfit) {
-    return vjp_exact_moduli(e, interval, grad, misfit);
+    return vjp_exact_moduli(e, interval, false, grad, misfit);
 }
 
 // The elastic form: the moduli gradient through pi = rho vp^2, u = rho vs^2
 // (readmod.c with L = 0) onto vp, vs, rho, [3][NY*NX*NZ].
 extern "C" int ifosb_vjp_exact(ifosb_engine *e, int interval, double *grad, double *misfit) {
     if (!e || !misfit || interval < 1) return IFOSB_EARG;
-    const ifosb_params &p = e->p;
-    if (p.nmech != 0)
+    if (e->p.nmech != 0)
         return fail(e, IFOSB_EARG, "the (vp, vs, rho) form is elastic; ifosb_vjp_exact_moduli takes L > 0");
-    if (!grad) return vjp_exact_moduli(e, interval, nullptr, misfit);
-    const size_t n = (size_t)p.nx * p.ny * p.nz, ng = (size_t)(p.nx + 2) * (p.ny + 2) * (p.nz + 2);
-    std::vector<double> gm(5 * n);
-    int rc = vjp_exact_moduli(e, interval, gm.data(), misfit);
-    if (rc) return rc;
-    std::vector<float> rawh(3 * ng);
-    CU(cudaMemcpy(rawh.data(), e->d_mstage, rawh.size() * sizeof(float), cudaMemcpyDeviceToHost));
-    const int NX = p.nx, NY = p.ny, NZ = p.nz, GX = NX + 2, GZ = NZ + 2;
-    const float *rho = rawh.data(), *pi = rho + ng, *u = pi + ng;
-    const double *fr = gm.data(), *fp = fr + n, *fu = fp + n;
-    for (int j = 1; j <= NY; ++j)
-        for (int i = 1; i <= NX; ++i)
-            for (int k = 1; k <= NZ; ++k) {
-                const size_t m = ((size_t)(j - 1) * NX + (i - 1)) * NZ + (k - 1), c = ((size_t)j * GX + i) * GZ + k;
-                const double r = rho[c], vp = std::sqrt((double)pi[c] / r), vs = std::sqrt((double)u[c] / r);
-                grad[m] = fp[m] * 2.0 * r * vp;
-                grad[n + m] = fu[m] * 2.0 * r * vs;
-                grad[2 * n + m] = fr[m] + fp[m] * vp * vp + fu[m] * vs * vs;
-            }
-    return IFOSB_OK;
+    return vjp_exact_moduli(e, interval, true, grad, misfit);
 }
 
 // ---------------------------------------------------------------------------
