@@ -207,7 +207,10 @@ __global__ void __launch_bounds__(64 * VYB, 4) k_velocity_box(const __grid_const
             tma_prefetch5(&T.v, z, x, y, VX, s);
             tma_prefetch3(&T.rho, z, x, y);
         },
-        [&](int j) { psi_find(q, g, a.sl, ps, j, b.i, b.k); },
+        [&](int j) {
+            psi_find(q, g, a.sl, ps, j, b.i, b.k);
+            if (a.u) prefetch3(a.u + (long long)s * 3 * g.field + widx(g, j, b.i, b.k), g.field);
+        },
         [&](int j) { vel_quad<BACK>(a, M(sm, b.y, b.x, b.zq), q, nt, s, j, b.i, b.k, g.nz - b.k + 1, p0, p1); });
 }
 

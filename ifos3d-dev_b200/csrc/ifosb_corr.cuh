@@ -79,8 +79,8 @@ struct CorrBox {
 struct Set {
     float2 c[3], d[9];
 };
-template <bool P2>
-__device__ __forceinline__ void take(Set &s, const float *grp, const CorrArgs &a, int y, int x, int z) {
+template <bool P2, class Args>
+__device__ __forceinline__ void take(Set &s, const float *grp, const Args &a, int y, int x, int z) {
     using M = StrSm<CYB>;
     const M m(grp, 0, y, x, z);
     constexpr int I = M::vI(), J = M::vJ();
@@ -292,6 +292,92 @@ __global__ void __launch_bounds__(CTHR, 2) k_corr(const __grid_constant__ CorrBo
 #pragma unroll
     for (int c = 0; c < 2; ++c)
         if (c < nc) cell[c].store(a, m + c, n);
+}
+
+// The time-domain kernels' zero-lag correlations of one pair of steps (TdArgs): per shot
+// the two sets of running sums come as boxes, the velocities of the cell itself directly.
+struct TdBox {
+    CUtensorMap F, B;  // forward / adjoint running sums [shot][3][y][x][z], one field with its halo
+    TdArgs a;
+    int *tma_err;
+};
+template <bool P2>
+__global__ void __launch_bounds__(CTHR, 4) k_td_corr(const __grid_constant__ TdBox T) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ uint64_t full[2];
+    const TdArgs &a = T.a;
+    const Geo &g = a.g;
+    float *sm = reinterpret_cast<float *>(smem);
+    const int k0 = blockIdx.x * TZ + 1, i0 = blockIdx.y * TX + 1, j0 = blockIdx.z * CYB + 1;
+    const int z = (threadIdx.x & 15) * 2, x = (threadIdx.x >> 4) & 7, y = threadIdx.x >> 7;
+    const int k = k0 + z, i = i0 + x, j = j0 + y;
+    const int nc = i <= g.nx && j <= g.ny ? min(2, g.nz - k + 1) : 0;  // this thread's cells
+    auto issue = [&](int s, int q) {
+        const CUtensorMap *m = q ? &T.B : &T.F;
+        float *d = sm + q * CGRP;
+        mbar_expect_tx(&full[q], 4 * 3 * StrSm<CYB>::VN);
+        tma_load5(d, m, zc(k0) - HZ, xc(i0) - 2, yc_(j0) - 1, 0, s, &full[q]);
+        tma_load5(d + StrSm<CYB>::VS, m, zc(k0) - HZ, xc(i0) - 1, yc_(j0) - 2, 1, s, &full[q]);
+        tma_load5(d + 2 * StrSm<CYB>::VS, m, zc(k0) - HZ, xc(i0) - 1, yc_(j0) - 1, 2, s, &full[q]);
+    };
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2; ++q) mbar_init(&full[q], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        for (int q = 0; q < 2; ++q) issue(0, q);
+    }
+    __syncthreads();
+    const long long n = (long long)g.nx * g.ny * g.nz, F = g.field, m = ((long long)(j - 1) * g.nx + (i - 1)) * g.nz + (k - 1);
+    const long long c = widx(g, j, i, k);
+    double kr[2] = {0.0, 0.0}, kl[2] = {0.0, 0.0}, km[2] = {0.0, 0.0}, old[3][2];
+#pragma unroll
+    for (int w = 0; w < 2; ++w)  // on their way while the boxes land
+        if (w < nc) { old[0][w] = a.k[m + w]; old[1][w] = a.k[n + m + w]; old[2][w] = a.k[2 * n + m + w]; }
+    for (int s = 0; s < a.nshots; ++s) {
+        float2 vf[3], vb[3];
+        if (nc > 0) {
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                vf[q] = ld2(a.seg + (long long)s * a.seg_shot + q * F + c);
+                vb[q] = ld2(a.st + (long long)s * a.st_shot + q * F + c);
+            }
+        }
+        Set set[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            bool ok = mbar_wait(&full[q], s & 1, WAIT_LIMIT_NS);
+            if (!ok) atomicExch(T.tma_err, 1);
+            else if (nc > 0) take<P2>(set[q], sm + q * CGRP, a, y, x, z);
+            if (!__syncthreads_and(ok)) {  // no copy may still be landing when the CTA ends
+                if (threadIdx.x == 0)
+                    for (int w = 0; w < 2; ++w) mbar_wait(&full[w], (w < q ? s + (s + 1 < a.nshots) : s) & 1, WAIT_LIMIT_NS);
+                return;
+            }
+            if (threadIdx.x == 0 && s + 1 < a.nshots) issue(s + 1, q);
+        }
+#pragma unroll
+        for (int w = 0; w < 2; ++w) {
+            if (w >= nc) continue;
+            float fu[9], bu[9];
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                fu[q] = at2(set[0].d[q], w);
+                bu[q] = at2(set[1].d[q], w);
+            }
+            kr[w] += (double)at2(vf[0], w) * at2(vb[0], w) + (double)at2(vf[1], w) * at2(vb[1], w) +
+                     (double)at2(vf[2], w) * at2(vb[2], w);
+            kl[w] += ((double)fu[0] + fu[4] + fu[8]) * ((double)bu[0] + bu[4] + bu[8]);
+            km[w] += 2.0 * ((double)fu[0] * bu[0] + (double)fu[4] * bu[4] + (double)fu[8] * bu[8]) +
+                     ((double)fu[1] + fu[3]) * ((double)bu[1] + bu[3]) + ((double)fu[2] + fu[6]) * ((double)bu[2] + bu[6]) +
+                     ((double)fu[5] + fu[7]) * ((double)bu[5] + bu[7]);
+        }
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+        if (w < nc) {
+            a.k[m + w] = old[0][w] + kr[w];
+            a.k[n + m + w] = old[1][w] + kl[w];
+            a.k[2 * n + m + w] = old[2][w] + km[w];
+        }
 }
 
 }  // namespace ifosb

@@ -801,6 +801,7 @@ static void fill_common(ifosb_engine *e, Loop &L) {
     va.cpg = sa.cpg = e->d_cpg;
     va.rho = e->d_rho_w;
     va.fast_div = e->cpml_div && e->rho_div;
+    va.dt = p.dt;
     sa.fast_div = e->cpml_div && div_range(p.dx) && div_range(p.dy) && div_range(p.dz);
     sa.unif_tau = e->unif_tau;
     sa.utaus = e->utaus; sa.utaup = e->utaup; sa.uts_avg = e->uts_avg;
@@ -989,10 +990,18 @@ static int attach_ring(ifosb_engine *e, Loop &L) {
     return IFOSB_OK;
 }
 
+// The running sums the velocity kernel keeps, and the segment step it writes besides.
+static void set_sums(Loop &L, float *u, float *seg, long long seg_shot) {
+    L.va.u = L.vt.a.u = u;
+    L.va.useg = L.vt.a.useg = seg;
+    L.va.useg_shot = L.vt.a.useg_shot = seg_shot;
+}
+
 // The kernel arguments of a planned loop, once va and sa are complete.
 static int finish_plan(ifosb_engine *e, Loop &L) {
     L.vt.a = L.va;
     L.stt.a = L.sa;
+    if (L.td.K) set_sums(L, L.td.uf, nullptr, 0);
     L.da.g = e->g;
     L.da.dft = L.dft;
     L.da.dft_shot = e->dft_shot;
@@ -1143,20 +1152,15 @@ static bool td_layout(const ifosb_engine *e, int nshots, int interval, TdLayout 
     return true;
 }
 
-static void td_integrate(ifosb_engine *e, int nshots, float *u, const float *st, float *seg, size_t seg_shot) {
-    k_td_integrate<<<dim3(2 * 148, nshots), 256, 0, e->stream>>>(u, st, e->st_shot, e->g.field, nshots, e->p.dt, seg,
-                                                                 (long long)seg_shot);
-}
-
 static void hook_copy(ifosb_engine *e, void *dst, const void *src, size_t words) {
     const cudaError_t r = cudaMemcpyAsync(dst, src, words * sizeof(float), cudaMemcpyDeviceToDevice, e->stream);
     if (r != cudaSuccess && e->hook_err == cudaSuccess) e->hook_err = r;
 }
 
-// after forward step nt of an armed forward (the engine's own state)
+// after forward step nt of an armed forward (the engine's own state; its velocity kernel
+// keeps the running sums)
 static void td_hook(ifosb_engine *e, const Loop &L, int nt) {
     const TdHook &t = L.td;
-    td_integrate(e, L.nshots, t.uf, e->d_state, nullptr, 0);
     if (nt % t.K == 0 && nt / t.K < t.nseg) {
         float *c = t.ckp + (size_t)(nt / t.K - 1) * t.ck;
         hook_copy(e, c, e->d_state, t.ssz);
@@ -1662,12 +1666,28 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
             CU(cudaStreamSynchronize(e->stream));  // init lives on the host stack
         }
         const int nb = 2 * 148, tb = 256;
-        const dim3 grd_c((p.nz + BX - 1) / BX, (p.nx + BY - 1) / BY, p.ny);
-        auto integrate = [&](float *u, const float *st, float *seg) { td_integrate(e, nshots, u, st, seg, seg_shot); };
+        const dim3 grd_c((p.nz + TZ - 1) / TZ, (p.nx + TX - 1) / TX, (p.ny + CYB - 1) / CYB);
+        const size_t smem_c = 4 * (size_t)2 * CGRP;
+        smem_set(p2 ? (const void *)k_td_corr<true> : (const void *)k_td_corr<false>, smem_c);
+        TdBox tdb;
+        std::memset(static_cast<void *>(&tdb), 0, sizeof(tdb));
+        tdb.tma_err = e->d_tma_err;
+        auto sums_map = [&](CUtensorMap *m, float *base, long long shot) {
+            const Geo &g = e->g;
+            const cuuint64_t dims[5] = {(cuuint64_t)g.pz, (cuuint64_t)g.px, (cuuint64_t)(p.ny + 5), 3, (cuuint64_t)nshots};
+            const cuuint64_t str[4] = {(cuuint64_t)g.pz * 4, (cuuint64_t)g.plane * 4, (cuuint64_t)g.field * 4, (cuuint64_t)shot * 4};
+            const cuuint32_t box[5] = {WZ, XH, CYB + 3, 1, 1};
+            return encode(m, base, 5, dims, str, box);
+        };
+        if (!sums_map(&tdb.B, ub, 3 * e->g.field) || !sums_map(&tdb.F, segb + 3 * e->g.field, (long long)seg_shot))
+            return fail(e, IFOSB_ECUDA, "tensor map of the running sums");
         set_slots(Lf, 0, 0);
         set_slots(La, 0, 0);
         auto enqueue = [&]() {
             cudaMemsetAsync(dk, 0, (size_t)4 * n * sizeof(double), e->stream);
+            cudaMemsetAsync(segb, 0, (size_t)K * seg_shot * nshots * sizeof(float), e->stream);  // halos
+            set_sums(Lf, uf, nullptr, 0);
+            set_sums(La, ub, nullptr, 0);
             if (!have_ck) {
                 // 1. the forward again, a checkpoint after steps K, 2K, ... and the sums at NT
                 cudaMemsetAsync(st2, 0, ss * sizeof(float), e->stream);
@@ -1675,7 +1695,6 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
                 cudaMemsetAsync(uf, 0, us * sizeof(float), e->stream);
                 for (int nt = 1; nt <= NT; ++nt) {
                     td_step(e, Lf, nt);
-                    integrate(uf, st2, nullptr);
                     if (nt % K == 0 && nt / K < nseg) {
                         float *c = ckp + (size_t)(nt / K - 1) * ck;
                         hook_copy(e, c, st2, ss);
@@ -1703,20 +1722,20 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
                     hook_copy(e, uf, c + ss + ps, us);
                 }
                 for (int m = a0; m <= a1; ++m) {  // v and U of each step go to the segment in the same pass
+                    set_sums(Lf, uf, segb + (size_t)(m - a0) * seg_shot * nshots, (long long)seg_shot);
                     td_step(e, Lf, m);
-                    integrate(uf, st2, segb + (size_t)(m - a0) * seg_shot * nshots);
                 }
                 for (int m = a1; m >= a0; --m, ++ntb) {  // adjoint steps P-a1 .. P-a0, in order
                     td_step(e, La, ntb);
-                    integrate(ub, e->d_state, nullptr);
                     ta.seg = segb + (size_t)(m - a0) * seg_shot * nshots;
-                    if (p2) k_td_corr<true><<<grd_c, dim3(BX, BY), 0, e->stream>>>(ta);
-                    else k_td_corr<false><<<grd_c, dim3(BX, BY), 0, e->stream>>>(ta);
+                    tdb.a = ta;
+                    sums_map(&tdb.F, const_cast<float *>(ta.seg) + 3 * e->g.field, (long long)seg_shot);
+                    if (p2) k_td_corr<true><<<grd_c, CTHR, smem_c, e->stream>>>(tdb);
+                    else k_td_corr<false><<<grd_c, CTHR, smem_c, e->stream>>>(tdb);
                 }
             }
             for (; ntb <= NT; ++ntb) {  // adjoint steps past P-1 meet forward steps before the first (zero)
                 td_step(e, La, ntb);
-                integrate(ub, e->d_state, nullptr);
             }
             k_td_dc<<<nb, tb, 0, e->stream>>>(ta, uf_end);
         };

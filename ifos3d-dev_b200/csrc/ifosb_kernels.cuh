@@ -70,18 +70,6 @@ struct Pt {
 };
 enum { PT_EXPLOSIVE = 1, PT_ADJOINT = 6, PT_RECEIVER = 7 };
 
-// a / b rounded to nearest (IEEE), the same bits as the division operator. The
-// division's range check sends a zero dividend down its slow path (three times
-// the cost of a normal quotient), and a wavefield is zero ahead of its front, so
-// a zero dividend is handled here: q = 2^-24 / b has the sign of b, is finite for
-// every finite non-zero b (2^-24 / 2^-149 = 2^125), +-0 for b = +-inf or |b| near
-// FLT_MAX, inf for b = 0 and NaN for b = NaN; a * q is then exactly 0 / b
-// (+-0 with the sign of a xor b, NaN for b = 0 or NaN).
-__device__ __forceinline__ float div_rn(float a, float b) {
-    const bool z = a == 0.f;
-    const float q = __fdiv_rn(z ? 0x1p-24f : a, b);
-    return z ? __fmul_rn(a, q) : q;
-}
 // z-face slab indices differ between the lanes of a warp; the constant cache would
 // serialise them, L1 serves them in one pass
 __device__ __forceinline__ float CPG(const float *cpg, int row, int h) { return __ldg(cpg + row * 2 * MAXFW + h - 1); }
@@ -124,6 +112,11 @@ struct VelArgs {
     const float *vin;     // velocities before the step [shot][3][field], and where the new ones go
     float *vout;          // (a slot of the velocity ring; the same place without one)
     long long vin_shot, vout_shot;
+    // time-domain mode: the running sums U += v dt of the new velocities [shot][3][field] (null:
+    // none), and where v and U go besides [shot][6][field] (null: nowhere)
+    float *u, *useg;
+    long long useg_shot;
+    float dt;
     const float *md;      // model base
     const float *rho;     // rho in field layout (with matcopy's ghost layers)
     float *psi;           // PML memory base (shot 0)
@@ -285,38 +278,6 @@ __global__ void __launch_bounds__(128, 8) k_dft(const __grid_constant__ DftArgs 
 }
 
 // ---------------------------------------------------------------------------
-// x / h with the division operator's bits: for a power-of-two spacing the exact
-// reciprocal (x * (1/h) == x / h for h = 2^k), else div_rn (no slow path for the
-// zero dividends of a field the wave has not reached)
-template <bool P2>
-__device__ __forceinline__ float dvh(float x, float h, float ih) {
-    return P2 ? __fmul_rn(x, ih) : div_rn(x, h);
-}
-
-// d: a float[9]; DX.. the spacings, IX.. their
-// reciprocals (used with P2)
-template <bool P2, class D>
-__device__ __forceinline__ void dft_derivs(const float *X, const float *Y, const float *Z, long long c, long long dI,
-                                           long long dJ, float b1, float b2, float DX, float DY, float DZ, float IX,
-                                           float IY, float IZ, D d) {
-    d[0] = dvh<P2>(b1 * (X[c] - X[c - dI]) + b2 * (X[c + dI] - X[c - 2 * dI]), DX, IX);
-    d[1] = dvh<P2>(b1 * (X[c + dJ] - X[c]) + b2 * (X[c + 2 * dJ] - X[c - dJ]), DY, IY);
-    d[2] = dvh<P2>(b1 * (X[c + 1] - X[c]) + b2 * (X[c + 2] - X[c - 1]), DZ, IZ);
-    d[3] = dvh<P2>(b1 * (Y[c + dI] - Y[c]) + b2 * (Y[c + 2 * dI] - Y[c - dI]), DX, IX);
-    d[4] = dvh<P2>(b1 * (Y[c] - Y[c - dJ]) + b2 * (Y[c + dJ] - Y[c - 2 * dJ]), DY, IY);
-    d[5] = dvh<P2>(b1 * (Y[c + 1] - Y[c]) + b2 * (Y[c + 2] - Y[c - 1]), DZ, IZ);
-    d[6] = dvh<P2>(b1 * (Z[c + dI] - Z[c]) + b2 * (Z[c + 2 * dI] - Z[c - dI]), DX, IX);
-    d[7] = dvh<P2>(b1 * (Z[c + dJ] - Z[c]) + b2 * (Z[c + 2 * dJ] - Z[c - dJ]), DY, IY);
-    d[8] = dvh<P2>(b1 * (Z[c] - Z[c - 1]) + b2 * (Z[c + 1] - Z[c - 2]), DZ, IZ);
-}
-
-// The same pointer, hidden from the optimiser (an empty asm that "changes" it).
-__device__ __forceinline__ const float *opaque(const float *p) {
-    asm volatile("" : "+l"(p));
-    return p;
-}
-
-// ---------------------------------------------------------------------------
 // Time-domain gradient kernels (the optional checkpoint/recompute mode). For a
 // forward step n and the adjoint step m = P - n, P = TIME / DT (TIME = (NT-1) DT
 // after ifos3d.c:177), the pair whose discfourier phases agree (t_f - t_b =
@@ -338,41 +299,6 @@ struct TdArgs {
     double *k;             // [4][NY][NX][NZ]: rho, lambda, mu, dc
 };
 
-// One thread per interior cell: blocks of BX (z) x BY (x) cells, one plane each
-// (grid ceil(NZ/BX) x ceil(NX/BY) x NY). (A variant that marched 1-16 planes per
-// block with the x/z neighbours staged in shared memory and the y neighbours in
-// registers ran 1.5-2.2 times slower at 128^3: fewer loads, but a barrier between
-// each plane's loads and its arithmetic.)
-template <bool P2>
-__global__ void __launch_bounds__(BX *BY, 4) k_td_corr(TdArgs a) {
-    const Geo &g = a.g;
-    const int k = blockIdx.x * BX + threadIdx.x + 1, i = blockIdx.y * BY + threadIdx.y + 1, j = blockIdx.z + 1;
-    if (k > g.nz || i > g.nx) return;
-    const long long n = (long long)g.nx * g.ny * g.nz, F = g.field, dI = g.pz, dJ = g.plane;
-    {
-        const long long m = ((long long)(j - 1) * g.nx + (i - 1)) * g.nz + (k - 1);
-        const long long c = widx(g, j, i, k);
-        double kr = 0.0, kl = 0.0, km = 0.0;
-        for (int s = 0; s < a.nshots; ++s) {
-            const float *vb = a.st + (long long)s * a.st_shot, *ub = a.ub + (long long)s * 3 * F;
-            const float *vf = a.seg + (long long)s * a.seg_shot, *uf = vf + 3 * F;
-            kr += (double)vf[c] * vb[c] + (double)vf[F + c] * vb[F + c] + (double)vf[2 * F + c] * vb[2 * F + c];
-            float fu[9], bu[9];
-            const float *p0 = opaque(uf + c), *p1 = opaque(uf + F + c), *p2 = opaque(uf + 2 * F + c);
-            dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, fu);
-            p0 = opaque(ub + c); p1 = opaque(ub + F + c); p2 = opaque(ub + 2 * F + c);
-            dft_derivs<P2>(p0, p1, p2, 0, dI, dJ, a.b1, a.b2, a.rdx, a.rdy, a.rdz, a.ihx, a.ihy, a.ihz, bu);
-            kl += ((double)fu[0] + fu[4] + fu[8]) * ((double)bu[0] + bu[4] + bu[8]);
-            km += 2.0 * ((double)fu[0] * bu[0] + (double)fu[4] * bu[4] + (double)fu[8] * bu[8]) +
-                  ((double)fu[1] + fu[3]) * ((double)bu[1] + bu[3]) + ((double)fu[2] + fu[6]) * ((double)bu[2] + bu[6]) +
-                  ((double)fu[5] + fu[7]) * ((double)bu[5] + bu[7]);
-        }
-        a.k[m] += kr;
-        a.k[n + m] += kl;
-        a.k[2 * n + m] += km;
-    }
-}
-
 // The zero-frequency product of the two runs: sum_c U_f,c(NT) U_b,c(NT).
 __global__ void k_td_dc(TdArgs a, const float *uf_end) {
     const Geo &g = a.g;
@@ -386,35 +312,6 @@ __global__ void k_td_dc(TdArgs a, const float *uf_end) {
             d += (double)uf[c] * ub[c] + (double)uf[F + c] * ub[F + c] + (double)uf[2 * F + c] * ub[2 * F + c];
         }
         a.k[3 * n + m] += d;
-    }
-}
-
-// U += v * DT over the three velocity fields (whole padded fields) of shot
-// blockIdx.y, four floats at a time (a field is a multiple of 8 floats and every
-// base is 16-byte aligned), each component as the scalar u + v * dt. With seg
-// set, the step's v and new U also go to the shot's segment slot
-// (seg + s * seg_shot: [v 3F][U 3F]), in the same pass.
-__global__ void k_td_integrate(float *u, const float *st, long long st_shot, long long F, int nshots, float dt,
-                               float *seg, long long seg_shot) {
-    const int s = blockIdx.y;
-    if (s >= nshots) return;
-    const long long n4 = 3 * F / 4;
-    float4 *U = reinterpret_cast<float4 *>(u + (long long)s * 3 * F);
-    const float4 *S = reinterpret_cast<const float4 *>(st + (long long)s * st_shot);
-    float4 *SV = seg ? reinterpret_cast<float4 *>(seg + (long long)s * seg_shot) : nullptr;
-    float4 *SU = seg ? SV + n4 : nullptr;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n4; q += (long long)gridDim.x * blockDim.x) {
-        float4 x = U[q];
-        const float4 v = S[q];
-        x.x += v.x * dt;
-        x.y += v.y * dt;
-        x.z += v.z * dt;
-        x.w += v.w * dt;
-        U[q] = x;
-        if (SV) {
-            SV[q] = v;
-            SU[q] = x;
-        }
     }
 }
 

@@ -217,6 +217,21 @@ __device__ __forceinline__ void vel_quad(const VelArgs &a, const S &m, Psi &q, i
     st4n(V + VX * F, v[0], ncell);
     st4n(V + VY * F, v[1], ncell);
     st4n(V + VZ * F, v[2], ncell);
+    if (a.u) {
+        // U += v DT beside the update: one pass over U instead of a launch that reads the
+        // velocities again and, for a segment, writes what it has just read
+        float *U = a.u + (long long)s * 3 * F + widx(g, j, i, k);
+        const F4 u[3] = {ld4(U) + a.dt * v[0], ld4(U + F) + a.dt * v[1], ld4(U + 2 * F) + a.dt * v[2]};
+        float *G = a.useg ? a.useg + (long long)s * a.useg_shot + widx(g, j, i, k) : nullptr;
+#pragma unroll
+        for (int n = 0; n < 3; ++n) {
+            st4n(U + n * F, u[n], ncell);
+            if (G) {
+                st4n(G + n * F, v[n], ncell);
+                st4n(G + (3 + n) * F, u[n], ncell);
+            }
+        }
+    }
     if (j == a.probe_j && i == a.probe_i && a.probe_k >= k && a.probe_k < k + 4) {
 #pragma unroll
         for (int n = 0; n < 4; ++n)
