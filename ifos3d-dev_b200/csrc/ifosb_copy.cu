@@ -1,0 +1,158 @@
+// See ifosb_copy.h. The driver's own path for pageable memory is one thread that copies
+// through its staging buffer (12.7 GB/s up, 20 down, 4.6 down into fresh pages on a
+// 16-core host). With these: a 44 MB result into a fresh array 9.6 -> 3 ms, the five
+// fields of a 131x101x150 model 3.3 -> 1.5 ms, a model update at 128^3 (102 MB both ways)
+// 7.2 -> 5.7 ms.
+#include "ifosb_copy.h"
+
+#include <algorithm>
+#include <cstring>
+#include <mutex>
+#include <system_error>
+#include <thread>
+#include <vector>
+
+namespace ifosb {
+namespace {
+
+constexpr size_t CHUNK = 1 << 20;       // bytes of a pinned chunk
+constexpr int MAXT = 8, SLOTS = 2;      // threads, chunks each: 16 MB pinned at most
+constexpr size_t LEAST = 4 * CHUNK;     // smaller copies are left to the driver
+
+struct Pool {
+    std::mutex m;  // held through a copy: one at a time uses the chunks, others take the driver's path
+    int refs = 0, device = -1;
+    char *pin = nullptr;
+    cudaStream_t st[MAXT] = {};
+    cudaEvent_t start = nullptr, done[MAXT] = {}, slot[MAXT][SLOTS] = {};
+
+    void free_all() {
+        for (int t = 0; t < MAXT; ++t) {
+            if (st[t]) cudaStreamSynchronize(st[t]), cudaStreamDestroy(st[t]);
+            if (done[t]) cudaEventDestroy(done[t]);
+            for (cudaEvent_t e : slot[t])
+                if (e) cudaEventDestroy(e);
+            st[t] = nullptr;
+            done[t] = nullptr;
+            std::fill(slot[t], slot[t] + SLOTS, nullptr);
+        }
+        if (start) cudaEventDestroy(start);
+        start = nullptr;
+        if (pin) cudaFreeHost(pin);
+        pin = nullptr;
+        device = -1;
+    }
+    bool ready(int dev) {
+        if (pin) return device == dev;
+        bool ok = cudaHostAlloc((void **)&pin, CHUNK * MAXT * SLOTS, cudaHostAllocDefault) == cudaSuccess &&
+                  cudaEventCreateWithFlags(&start, cudaEventDisableTiming) == cudaSuccess;
+        for (int t = 0; ok && t < MAXT; ++t) {
+            ok = cudaStreamCreateWithFlags(&st[t], cudaStreamNonBlocking) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&done[t], cudaEventDisableTiming) == cudaSuccess;
+            for (int s = 0; ok && s < SLOTS; ++s)
+                ok = cudaEventCreateWithFlags(&slot[t][s], cudaEventDisableTiming) == cudaSuccess;
+        }
+        if (!ok) {
+            cudaGetLastError();
+            free_all();
+            return false;
+        }
+        device = dev;
+        return true;
+    }
+};
+Pool &pool() {
+    static Pool *p = new Pool;  // outlives every caller
+    return *p;
+}
+
+bool pageable(const void *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
+}  // namespace
+
+int host_parts(size_t bytes) {
+    const int cpus = (int)std::thread::hardware_concurrency();
+    return (int)std::max<size_t>(1, std::min<size_t>(std::min(MAXT, cpus / 2), bytes / (2 * CHUNK)));
+}
+
+void run_parts(int parts, const std::function<void(int)> &fn) {
+    std::vector<std::thread> th;
+    int next = 1;
+    try {
+        th.reserve((size_t)std::max(parts - 1, 0));
+        for (; next < parts; ++next) th.emplace_back(fn, next);
+    } catch (const std::exception &) {
+        // no more threads to be had: the caller does the rest
+    }
+    fn(0);
+    for (; next < parts; ++next) fn(next);
+    for (std::thread &t : th) t.join();
+}
+
+void host_copy_retain() {
+    std::lock_guard<std::mutex> l(pool().m);
+    ++pool().refs;
+}
+void host_copy_release() {
+    std::lock_guard<std::mutex> l(pool().m);
+    if (--pool().refs == 0) pool().free_all();
+}
+
+cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    Pool &p = pool();
+    const int parts = host_parts(bytes);
+    int dev = 0;
+    const bool up = bytes >= LEAST && parts > 1 && pageable(src), down = bytes >= LEAST && parts > 1 && !up && pageable(dst);
+    std::unique_lock<std::mutex> lock(p.m, std::defer_lock);
+    if (!(up != down) || (up && pageable(dst)) || cudaGetDevice(&dev) != cudaSuccess || !lock.try_lock() || !p.ready(dev))
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
+    cudaError_t err[MAXT] = {};
+    cudaError_t e = cudaEventRecord(p.start, st);
+    if (e != cudaSuccess) return e;
+    const size_t n = (bytes + CHUNK - 1) / CHUNK;
+    run_parts(parts, [&](int t) {
+        cudaError_t r = cudaSetDevice(dev);
+        if (r == cudaSuccess) r = cudaStreamWaitEvent(p.st[t], p.start, 0);
+        auto chunk = [&](size_t c) { return std::min(CHUNK, bytes - c * CHUNK); };
+        auto pinned = [&](int s) { return p.pin + ((size_t)t * SLOTS + s) * CHUNK; };
+        int s = 0;
+        if (up) {
+            for (size_t c = t; r == cudaSuccess && c < n; c += parts, s ^= 1) {
+                r = cudaEventSynchronize(p.slot[t][s]);  // the slot's last transfer
+                if (r != cudaSuccess) break;
+                std::memcpy(pinned(s), (const char *)src + c * CHUNK, chunk(c));
+                r = cudaMemcpyAsync((char *)dst + c * CHUNK, pinned(s), chunk(c), cudaMemcpyHostToDevice, p.st[t]);
+                if (r == cudaSuccess) r = cudaEventRecord(p.slot[t][s], p.st[t]);
+            }
+            if (r == cudaSuccess) r = cudaEventRecord(p.done[t], p.st[t]);
+        } else {
+            auto fetch = [&](size_t c, int q) {
+                r = cudaEventSynchronize(p.slot[t][q]);
+                if (r == cudaSuccess)
+                    r = cudaMemcpyAsync(pinned(q), (const char *)src + c * CHUNK, chunk(c), cudaMemcpyDeviceToHost, p.st[t]);
+                if (r == cudaSuccess) r = cudaEventRecord(p.slot[t][q], p.st[t]);
+            };
+            if (r == cudaSuccess && (size_t)t < n) fetch(t, 0);
+            for (size_t c = t; r == cudaSuccess && c < n; c += parts, s ^= 1) {
+                if (c + parts < n) fetch(c + parts, s ^ 1);
+                if (r == cudaSuccess) r = cudaEventSynchronize(p.slot[t][s]);
+                if (r == cudaSuccess) std::memcpy((char *)dst + c * CHUNK, pinned(s), chunk(c));
+            }
+        }
+        err[t] = r;
+    });
+    for (int t = 0; t < parts && e == cudaSuccess; ++t) {
+        e = err[t];
+        if (e == cudaSuccess && up) e = cudaStreamWaitEvent(st, p.done[t], 0);
+    }
+    return e;
+}
+
+}  // namespace ifosb

@@ -8,6 +8,7 @@
 // and replayed on later calls.
 #include "../../include/ifos_b200.h"
 #include "ifosb_kernels.cuh"
+#include "ifosb_copy.h"
 #include "ifosb_corr.cuh"
 #include "ifosb_vjp.cuh"
 
@@ -103,6 +104,7 @@ struct ifosb_engine {
     int nt_limit = 0;
     long long captures = 0;  // time-loop graphs captured (a replay reuses one)
     float *d_mstage = nullptr;  // ifosb_set_model's staging of the raw model (5 ghosted fields)
+    float *d_mraw = nullptr;    // and of one interior field to be wrapped
     float *d_smod = nullptr;    // free-surface moduli of plane j=1 [2][NX][NZ] (ifosb_set_surface_moduli)
     bool smod_on = false;
     // approximate Hessian: receivers' Green's-function DFT fields and the accumulated diagonal
@@ -215,6 +217,11 @@ static int dgrow(ifosb_engine *e, T **ptr, size_t *cap, size_t count) {
     return rc;
 }
 
+static uint32_t float_bits(float x) {
+    uint32_t b;
+    std::memcpy(&b, &x, sizeof(b));
+    return b;
+}
 static bool div_range(float b) { return b >= DIV_B_MIN && b <= DIV_B_MAX; }
 
 static void fd_coeffs(int fdcoeff, float *b1, float *b2) {
@@ -296,6 +303,7 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
         !(p->dy > 0.f) || !(p->dz > 0.f))
         return IFOSB_EARG;
     ifosb_engine *e = new ifosb_engine();
+    host_copy_retain();
     e->p = *p;
     e->max_shots = max_shots;
     e->max_nf = max_nf;
@@ -333,7 +341,7 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
         g.zfo = whole ? 0 : zb - far / 4 * 4;
         g.pzw = ((whole ? p->nz : zb + far % 4 + p->fw) + 3) / 4 * 4;
     }
-    if ((long long)g.nyc * max_shots > 65535) { delete e; return IFOSB_EARG; }
+    if ((long long)g.nyc * max_shots > 65535) { host_copy_release(); delete e; return IFOSB_EARG; }
     e->sl.sx = (long long)p->ny * 2 * p->fw * g.pz;
     e->sl.sy = (long long)2 * p->fw * p->nx * g.pz;
     e->sl.sz = (long long)p->ny * p->nx * g.pzw;
@@ -342,6 +350,7 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
     e->dft_shot = (long long)max_nf * 6 * g.field;
     if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess) {
         cudaGetLastError();
+        host_copy_release();
         delete e;
         return IFOSB_ECUDA;
     }
@@ -395,11 +404,12 @@ extern "C" void ifosb_destroy(ifosb_engine *e) {
                     e->d_trig_b, e->d_voff, e->d_soff, e->d_vpts, e->d_spts, e->d_amp, e->d_tma_err, e->d_cpg,
                     e->d_mstage, e->d_green, e->d_gsig, e->d_hess, e->d_sec2, e->d_voff_t, e->d_soff_t,
                     e->d_voff_a, e->d_vpts_t, e->d_spts_t, e->d_vpts_a, e->d_amp_t, e->d_gradq, e->d_smod,
-                    e->d_td_blk, e->d_td_k, e->d_ring};
+                    e->d_td_blk, e->d_td_k, e->d_ring, e->d_mraw};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (cudaEvent_t ev : e->events) cudaEventDestroy(ev);
     if (e->own_stream) cudaStreamDestroy(e->own_stream);
+    host_copy_release();
     delete e;
 }
 
@@ -496,35 +506,95 @@ extern "C" int ifosb_set_cpml(ifosb_engine *e, const float *coeff) {
     return IFOSB_OK;
 }
 
-extern "C" int ifosb_set_model(ifosb_engine *e, const float *rho, const float *pi, const float *u, const float *taus,
-                               const float *taup, const float *eta) {
+// Model values as positive finite floats: their bits lie between 1 and those of the
+// largest float; of rho also whether every value is in the division's range (an average
+// of two then is too). Large models are looked through by a few threads.
+static bool model_ok(const float *a, size_t n, bool &in_range) {
+    const int parts = host_parts(n * sizeof(float));
+    std::vector<unsigned char> bad(parts, 0), out(parts, 0);
+    const uint32_t lo = float_bits(DIV_B_MIN), hi = float_bits(DIV_B_MAX);
+    run_parts(parts, [&](int t) {
+        const size_t q1 = n * (t + 1) / parts;
+        uint32_t b = 0, o = 0;
+        for (size_t q = n * t / parts; q < q1; ++q) {
+            const uint32_t v = float_bits(a[q]);
+            b |= v - 1u >= 0x7f7fffffu;
+            o |= (uint32_t)(v < lo) | (uint32_t)(v > hi);
+        }
+        bad[t] = b != 0;
+        out[t] = o != 0;
+    });
+    in_range = std::find(out.begin(), out.end(), 1) == out.end();
+    return std::find(bad.begin(), bad.end(), 1) == bad.end();
+}
+static bool all_equal(const float *a, size_t n) {
+    const int parts = host_parts(n * sizeof(float));
+    std::vector<unsigned char> other(parts, 0);
+    run_parts(parts, [&](int t) {
+        const size_t q1 = n * (t + 1) / parts;
+        for (size_t q = n * t / parts; q < q1 && !other[t];) {
+            const size_t e = std::min(q1, q + 4096);
+            uint32_t d = 0;
+            for (; q < e; ++q) d |= (uint32_t)!(a[q] == a[0]);
+            other[t] = d != 0;
+        }
+    });
+    return std::find(other.begin(), other.end(), 1) == other.end();
+}
+
+// One interior field [NY][NX][NZ] with matcopy's ghost layer on one rank around it: a
+// periodic copy (receives from MPI_PROC_NULL leave the buffer untouched).
+__global__ void k_ghost_wrap(Geo g, const float *in, float *out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y, j = blockIdx.z;
+    if (k > g.nz + 1 || i > g.nx + 1) return;
+    const int jj = j == 0 ? g.ny : j > g.ny ? 1 : j, ii = i == 0 ? g.nx : i > g.nx ? 1 : i, kk = k == 0 ? g.nz : k > g.nz ? 1 : k;
+    out[((long long)j * (g.nx + 2) + i) * (g.nz + 2) + k] = in[((long long)(jj - 1) * g.nx + (ii - 1)) * g.nz + (kk - 1)];
+}
+
+// The model from the host's ghosted arrays, or from interior ones (wrapped on the device).
+static int set_model(ifosb_engine *e, const float *rho, const float *pi, const float *u, const float *taus, const float *taup,
+                     const float *eta, bool interior) {
     if (!e || !rho || !pi || !u) return IFOSB_EARG;
     const ifosb_params &p = e->p;
     if (p.nmech > 0 && (!taus || !taup || !eta)) return fail(e, IFOSB_EARG, "viscoelastic model needs taus, taup, eta");
     e->ngreen = 0;  // Green's functions belong to a model
-    const size_t ng = (size_t)(p.nx + 2) * (p.ny + 2) * (p.nz + 2);
-    float rlo = rho[0], rhi = rho[0];
-    for (size_t q = 0; q < ng; ++q) {
-        if (!(rho[q] > 0.f) || !(u[q] > 0.f) || !(pi[q] > 0.f) || !std::isfinite(rho[q]) || !std::isfinite(u[q]) ||
-            !std::isfinite(pi[q]))
-            return fail(e, IFOSB_EARG, "model value not positive and finite at ghosted index " + std::to_string(q));
-        rlo = std::min(rlo, rho[q]);
-        rhi = std::max(rhi, rho[q]);
+    const size_t ng = (size_t)(p.nx + 2) * (p.ny + 2) * (p.nz + 2), n = interior ? (size_t)p.nx * p.ny * p.nz : ng;
+    bool rho_range = false, other;
+    const bool ok = model_ok(rho, n, rho_range) & model_ok(pi, n, other) & model_ok(u, n, other);
+    if (!ok) {  // the first bad cell in the ghosted order
+        for (size_t q = 0; q < ng; ++q) {
+            size_t m = q;
+            if (interior) {
+                auto wrap = [](size_t x, int N) { return x == 0 ? (size_t)N - 1 : x > (size_t)N ? 0 : x - 1; };
+                const size_t k = wrap(q % (p.nz + 2), p.nz), i = wrap(q / (p.nz + 2) % (p.nx + 2), p.nx),
+                             j = wrap(q / ((size_t)(p.nz + 2) * (p.nx + 2)), p.ny);
+                m = (j * p.nx + i) * p.nz + k;
+            }
+            if (!(rho[m] > 0.f) || !(u[m] > 0.f) || !(pi[m] > 0.f) || !std::isfinite(rho[m]) || !std::isfinite(u[m]) ||
+                !std::isfinite(pi[m]))
+                return fail(e, IFOSB_EARG, "model value not positive and finite at ghosted index " + std::to_string(q));
+        }
     }
-    e->rho_div = rlo >= DIV_B_MIN && rhi <= DIV_B_MAX;  // and so is every average of two
     for (int l = 0; l < p.nmech; ++l)
         if (!std::isfinite(eta[l])) return fail(e, IFOSB_EARG, "eta not finite");
     if (!e->d_mstage) {  // staging for the raw model, kept for the engine's lifetime
         const int rc = dalloc(e, &e->d_mstage, ng * 5);
         if (rc) return rc;
     }
+    if (interior && !e->d_mraw) {
+        const int rc = dalloc(e, &e->d_mraw, n);
+        if (rc) return rc;
+    }
+    e->rho_div = rho_range;
     float *tmp = e->d_mstage;
-    CU(cudaMemcpyAsync(tmp, rho, ng * sizeof(float), cudaMemcpyHostToDevice, e->stream));
-    CU(cudaMemcpyAsync(tmp + ng, pi, ng * sizeof(float), cudaMemcpyHostToDevice, e->stream));
-    CU(cudaMemcpyAsync(tmp + 2 * ng, u, ng * sizeof(float), cudaMemcpyHostToDevice, e->stream));
-    if (p.nmech > 0) {
-        CU(cudaMemcpyAsync(tmp + 3 * ng, taus, ng * sizeof(float), cudaMemcpyHostToDevice, e->stream));
-        CU(cudaMemcpyAsync(tmp + 4 * ng, taup, ng * sizeof(float), cudaMemcpyHostToDevice, e->stream));
+    const float *src[5] = {rho, pi, u, taus, taup};
+    for (int q = 0; q < (p.nmech > 0 ? 5 : 3); ++q) {
+        if (!interior) {
+            CU(host_copy(tmp + q * ng, src[q], ng * sizeof(float), e->stream));
+            continue;
+        }
+        CU(host_copy(e->d_mraw, src[q], n * sizeof(float), e->stream));
+        k_ghost_wrap<<<dim3((p.nz + 2 + 31) / 32, (p.nx + 2 + 3) / 4, p.ny + 2), dim3(32, 4), 0, e->stream>>>(e->g, e->d_mraw, tmp + q * ng);
     }
     AvArgs a{};
     a.g = e->g;
@@ -543,9 +613,7 @@ extern "C" int ifosb_set_model(ifosb_engine *e, const float *rho, const float *p
     // staggered averages are one value too and the kernels take scalars
     e->unif_tau = false;
     if (p.nmech > 0) {
-        bool u = true;
-        for (size_t q = 1; q < ng && u; ++q) u = taus[q] == taus[0] && taup[q] == taup[0];
-        if (u) {
+        if (all_equal(taus, n) && all_equal(taup, n)) {
             const float t = taus[0];
             e->unif_tau = true;
             e->utaus = t;
@@ -556,6 +624,16 @@ extern "C" int ifosb_set_model(ifosb_engine *e, const float *rho, const float *p
     e->have_model = true;
     e->fwd_ok = e->res_ok = e->adj_ok = false;
     return IFOSB_OK;
+}
+
+extern "C" int ifosb_set_model(ifosb_engine *e, const float *rho, const float *pi, const float *u, const float *taus,
+                               const float *taup, const float *eta) {
+    return set_model(e, rho, pi, u, taus, taup, eta, false);
+}
+
+extern "C" int ifosb_set_model_interior(ifosb_engine *e, const float *rho, const float *pi, const float *u, const float *taus,
+                                        const float *taup, const float *eta) {
+    return set_model(e, rho, pi, u, taus, taup, eta, true);
 }
 
 // The elastic free surface's own moduli: the reference's step-length forwards
@@ -1423,7 +1501,7 @@ extern "C" int ifosb_residual(ifosb_engine *e, const float *obs, double *misfit_
     const int nshots = e->nshots, ntr = e->ntr, ns = e->ns;
     const size_t n = (size_t)nshots * 3 * ntr * ns;
     // obs may be host or device memory (unified addressing picks the copy's direction)
-    CU(cudaMemcpyAsync(e->d_obs, obs, n * sizeof(float), cudaMemcpyDefault, e->stream));
+    CU(host_copy(e->d_obs, obs, n * sizeof(float), e->stream));
     const int nthr = nshots * 3 * ntr;
     k_residual<<<(nthr + 127) / 128, 128, 0, e->stream>>>(e->d_sec, e->d_obs, e->d_diff, e->d_part, nshots, ntr, ns, e->p.dt);
     k_misfit<<<nshots, 32, 0, e->stream>>>(e->d_part, e->d_misfit, 3 * ntr);
@@ -1757,7 +1835,7 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
         if (e->hook_err != cudaSuccess)
             return fail(e, IFOSB_ECUDA, std::string("time-domain copies: ") + cudaGetErrorString(e->hook_err));
         if ((r = check_unstable(e, nshots))) return r;
-        CU(cudaMemcpyAsync(kernels, dk, (size_t)4 * n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+        CU(host_copy(kernels, dk, (size_t)4 * n * sizeof(double), e->stream));
         CU(cudaStreamSynchronize(e->stream));
         // the checkpoints stay in the block (the segments only read them): a repeat
         // call for this forward starts from them
@@ -1943,7 +2021,7 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *g
         k64_fold<<<grd3, blk3, 0, e->stream>>>(g, gr, md, raw, L, chain, fold);
         int r;
         if ((r = check_launch(e, "exact VJP gradient"))) return r;
-        CU(cudaMemcpyAsync(gmod, fold, (size_t)nq * n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+        CU(host_copy(gmod, fold, (size_t)nq * n * sizeof(double), e->stream));
         CU(cudaStreamSynchronize(e->stream));
         return IFOSB_OK;
     };
@@ -2075,7 +2153,7 @@ extern "C" int ifosb_get_hessian(ifosb_engine *e, float *hess) {
         std::memset(hess, 0, n * sizeof(float));
         return IFOSB_OK;
     }
-    CU(cudaMemcpyAsync(hess, e->d_hess, n * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
+    CU(host_copy(hess, e->d_hess, n * sizeof(float), e->stream));
     CU(cudaStreamSynchronize(e->stream));
     return IFOSB_OK;
 }
@@ -2094,7 +2172,7 @@ extern "C" int ifosb_get_gradient_q(ifosb_engine *e, double *gradq) {
     if (!e || !gradq) return IFOSB_EARG;
     if (!e->d_gradq) return fail(e, IFOSB_ESTATE, "the Q gradient needs a viscoelastic engine (nmech > 0)");
     const size_t n = (size_t)2 * e->p.nx * e->p.ny * e->p.nz;
-    CU(cudaMemcpyAsync(gradq, e->d_gradq, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+    CU(host_copy(gradq, e->d_gradq, n * sizeof(double), e->stream));
     CU(cudaStreamSynchronize(e->stream));
     return IFOSB_OK;
 }
@@ -2103,8 +2181,8 @@ extern "C" int ifosb_get_gradient(ifosb_engine *e, float *grad, double *grad64) 
     if (!e) return IFOSB_EARG;
     const size_t n = (size_t)3 * e->p.nx * e->p.ny * e->p.nz;
     // host or device destinations (unified addressing)
-    if (grad) CU(cudaMemcpyAsync(grad, e->d_grad, n * sizeof(float), cudaMemcpyDefault, e->stream));
-    if (grad64) CU(cudaMemcpyAsync(grad64, e->d_grad64, n * sizeof(double), cudaMemcpyDefault, e->stream));
+    if (grad) CU(host_copy(grad, e->d_grad, n * sizeof(float), e->stream));
+    if (grad64) CU(host_copy(grad64, e->d_grad64, n * sizeof(double), e->stream));
     CU(cudaStreamSynchronize(e->stream));
     return IFOSB_OK;
 }

@@ -10,12 +10,15 @@
 // one final block), so results are deterministic. The elementwise model update
 // keeps the reference's float/double expressions and is bit-identical to it.
 #include "../../include/ifos_b200.h"
+#include "ifosb_copy.h"
 
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <string>
 #include <vector>
+
+using namespace ifosb;
 
 namespace {
 
@@ -347,6 +350,7 @@ extern "C" int ifosb_optim_create(int nx, int ny, int nz, int numpar, int bfgsnu
     o->numpar = numpar;
     o->bfgsnum = bfgsnum;
     o->n = (long long)nx * ny * nz;
+    host_copy_retain();
     const long long n = o->n, nn = (long long)numpar * n, mg = (long long)(nx + 2) * (ny + 2) * (nz + 2);
     auto alloc = [&](void **p, size_t bytes) { return cudaMalloc(p, bytes) == cudaSuccess; };
     bool ok = alloc((void **)&o->d_grad, sizeof(float) * 3 * n) && alloc((void **)&o->d_prior, sizeof(float) * 6 * n) &&
@@ -379,6 +383,7 @@ extern "C" void ifosb_optim_destroy(ifosb_optim *o) {
                     (void *)o->d_part, (void *)o->d_sc, (void *)o->d_out, (void *)o->d_max, (void *)o->d_model})
         if (p) cudaFree(p);
     if (o->stream) cudaStreamDestroy(o->stream);
+    host_copy_release();
     delete o;
 }
 
@@ -394,7 +399,7 @@ extern "C" int ifosb_conjugate(ifosb_optim *o, float *grad, int cdf, double *bet
     if (!o || !grad) return IFOSB_EARG;
     const long long n = o->n;
     double *d_beta = o->d_sc + 2 * o->bfgsnum + 4;
-    OCU(cudaMemcpyAsync(o->d_grad, grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(o->d_grad, grad, sizeof(float) * 3 * n, o->stream));
     if (cdf == 1) {  // conjugategrad.c:43-56: both priors start from this gradient
         OCU(cudaMemcpyAsync(o->d_prior, o->d_grad, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, o->stream));
         OCU(cudaMemcpyAsync(o->d_prior + 3 * n, o->d_grad, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, o->stream));
@@ -403,7 +408,7 @@ extern "C" int ifosb_conjugate(ifosb_optim *o, float *grad, int cdf, double *bet
         k_final<<<1, 32, 0, o->stream>>>(o->d_part, 6, o->d_out);
         k_cg_beta<<<1, 32, 0, o->stream>>>(o->d_out, cdf, d_beta);
         k_cg_dir<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, o->d_prior + 3 * n, d_beta, n);
-        OCU(cudaMemcpyAsync(grad, o->d_grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream));
+        OCU(host_copy(grad, o->d_grad, sizeof(float) * 3 * n, o->stream));
     }
     int rc = finish(o);
     if (rc) return rc;
@@ -426,7 +431,7 @@ extern "C" int ifosb_lbfgs_savegrad(ifosb_optim *o, const float *grad) {
     if (!o || !grad) return IFOSB_EARG;
     if (o->bfgsnum < 1) return ofail(o, IFOSB_ESTATE, "optimiser created without L-BFGS history");
     const long long nn = (long long)o->numpar * o->n;
-    OCU(cudaMemcpyAsync(o->d_grad, grad, sizeof(float) * nn, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(o->d_grad, grad, sizeof(float) * nn, o->stream));
     k_copy_f2d<<<RBLK, RTHR, 0, o->stream>>>(o->d_y, o->d_grad, nn);  // lbfgs_save.c:31-52: slot 1
     return finish(o);
 }
@@ -441,7 +446,7 @@ extern "C" int ifosb_lbfgs(ifosb_optim *o, float *grad, int it_group) {
     if (m < 1) m = 1;
     auto S = [&](int w) { return o->d_s + (long long)(w - 1) * nn; };
     auto Y = [&](int w) { return o->d_y + (long long)(w - 1) * nn; };
-    OCU(cudaMemcpyAsync(o->d_grad, grad, sizeof(float) * nn, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(o->d_grad, grad, sizeof(float) * nn, o->stream));
     int w = slot(it_group - 1, B);
     k_lb_start<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, Y(w), o->d_q, nn);
     k_dot2<<<RBLK, RTHR, 0, o->stream>>>(Y(w), S(w), nn, o->d_part);
@@ -460,7 +465,7 @@ extern "C" int ifosb_lbfgs(ifosb_optim *o, float *grad, int it_group) {
         k_axpy<<<RBLK, RTHR, 0, o->stream>>>(o->d_q, S(w), sc + 2 * B + 1, nn);
     }
     k_lb_end<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, Y(slot(it_group, B)), o->d_q, nn);
-    OCU(cudaMemcpyAsync(grad, o->d_grad, sizeof(float) * nn, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(grad, o->d_grad, sizeof(float) * nn, o->stream));
     return finish(o);
 }
 
@@ -470,10 +475,10 @@ extern "C" int ifosb_modelupdate(ifosb_optim *o, float *grad, float *rho, float 
     if (lbfgs && o->bfgsnum < 1) return ofail(o, IFOSB_ESTATE, "optimiser created without L-BFGS history");
     const long long n = o->n, mg = (long long)(o->nx + 2) * (o->ny + 2) * (o->nz + 2);
     float *drho = o->d_model, *dpi = o->d_model + mg, *du = o->d_model + 2 * mg;
-    OCU(cudaMemcpyAsync(o->d_grad, grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(drho, rho, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(dpi, pi, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(du, u, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(o->d_grad, grad, sizeof(float) * 3 * n, o->stream));
+    OCU(host_copy(drho, rho, sizeof(float) * mg, o->stream));
+    OCU(host_copy(dpi, pi, sizeof(float) * mg, o->stream));
+    OCU(host_copy(du, u, sizeof(float) * mg, o->stream));
     if (!lbfgs) {
         OCU(cudaMemsetAsync(o->d_max, 0, sizeof(unsigned) * 3, o->stream));
         k_absmax<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, n, o->d_max);
@@ -493,10 +498,10 @@ extern "C" int ifosb_modelupdate(ifosb_optim *o, float *grad, float *rho, float 
     a.numpar = o->numpar;
     a.s = lbfgs ? o->d_s + (long long)(slot(it_group, o->bfgsnum) - 1) * o->numpar * n : nullptr;
     k_modelupdate<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, drho, dpi, du, a);
-    if (!lbfgs) OCU(cudaMemcpyAsync(grad, o->d_grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(rho, drho, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(pi, dpi, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(u, du, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
+    if (!lbfgs) OCU(host_copy(grad, o->d_grad, sizeof(float) * 3 * n, o->stream));
+    OCU(host_copy(rho, drho, sizeof(float) * mg, o->stream));
+    OCU(host_copy(pi, dpi, sizeof(float) * mg, o->stream));
+    OCU(host_copy(u, du, sizeof(float) * mg, o->stream));
     return finish(o);
 }
 
@@ -617,12 +622,12 @@ extern "C" int ifosb_precon_grad(ifosb_optim *o, float *grad, int damptype, int 
     int rc = IFOSB_OK;
     cudaError_t ce = cudaMemcpyAsync(dt, hf.data(), sizeof(float) * nf, cudaMemcpyHostToDevice, o->stream);
     if (ce == cudaSuccess && ni) ce = cudaMemcpyAsync(di, hi.data(), sizeof(int) * ni, cudaMemcpyHostToDevice, o->stream);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(o->d_grad, grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream);
+    if (ce == cudaSuccess) ce = host_copy(o->d_grad, grad, sizeof(float) * 3 * n, o->stream);
     if (ce == cudaSuccess) {
         k_precon<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, a);
         ce = cudaGetLastError();
     }
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(grad, o->d_grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream);
+    if (ce == cudaSuccess) ce = host_copy(grad, o->d_grad, sizeof(float) * 3 * n, o->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(o->stream);
     if (ce != cudaSuccess) {
         o->err = std::string("precon_grad: ") + cudaGetErrorString(ce);
@@ -661,13 +666,13 @@ extern "C" int ifosb_constant_boundary(ifosb_optim *o, float *rho, float *pi, fl
     };
     const long long mg = (long long)(NX + 2) * (NY + 2) * (NZ + 2);
     float *drho = o->d_model, *dpi = o->d_model + mg, *du = o->d_model + 2 * mg;
-    OCU(cudaMemcpyAsync(drho, rho, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(dpi, pi, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(du, u, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(drho, rho, sizeof(float) * mg, o->stream));
+    OCU(host_copy(dpi, pi, sizeof(float) * mg, o->stream));
+    OCU(host_copy(du, u, sizeof(float) * mg, o->stream));
     for (const CbPhase &q : ph) k_cbound<<<RBLK, RTHR, 0, o->stream>>>(drho, dpi, du, NX, NZ, q);
-    OCU(cudaMemcpyAsync(rho, drho, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(pi, dpi, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
-    OCU(cudaMemcpyAsync(u, du, sizeof(float) * mg, cudaMemcpyDefault, o->stream));
+    OCU(host_copy(rho, drho, sizeof(float) * mg, o->stream));
+    OCU(host_copy(pi, dpi, sizeof(float) * mg, o->stream));
+    OCU(host_copy(u, du, sizeof(float) * mg, o->stream));
     return finish(o);
 }
 
@@ -697,14 +702,14 @@ extern "C" int ifosb_hess_apply(ifosb_optim *o, float *grad, const float *hess, 
     const long long n = o->n;
     float *dh = nullptr;
     OCU(cudaMalloc(&dh, sizeof(float) * 3 * n));
-    cudaError_t ce = cudaMemcpyAsync(dh, hess, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(o->d_grad, grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream);
+    cudaError_t ce = host_copy(dh, hess, sizeof(float) * 3 * n, o->stream);
+    if (ce == cudaSuccess) ce = host_copy(o->d_grad, grad, sizeof(float) * 3 * n, o->stream);
     if (ce == cudaSuccess) {
         k_hess_apply<<<RBLK, RTHR, 0, o->stream>>>(o->d_grad, dh, n, water[0], water[1], water[2], lbfgs ? 1 : 0, vp0,
                                                    vs0, rho0);
         ce = cudaGetLastError();
     }
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(grad, o->d_grad, sizeof(float) * 3 * n, cudaMemcpyDefault, o->stream);
+    if (ce == cudaSuccess) ce = host_copy(grad, o->d_grad, sizeof(float) * 3 * n, o->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(o->stream);
     cudaFree(dh);
     if (ce != cudaSuccess) {

@@ -73,6 +73,7 @@ def lib():
             "ifosb_device_bytes": (C.c_longlong, [vp]),
             "ifosb_set_cpml": (C.c_int, [vp, vp]),
             "ifosb_set_model": (C.c_int, [vp, vp, vp, vp, vp, vp, vp]),
+            "ifosb_set_model_interior": (C.c_int, [vp, vp, vp, vp, vp, vp, vp]),
             "ifosb_set_receivers": (C.c_int, [vp, C.c_int, vp]),
             "ifosb_set_frequencies": (C.c_int, [vp, C.c_int, vp, C.c_int]),
             "ifosb_forward": (C.c_int, [vp, C.c_int, C.POINTER(Shot), vp]),
@@ -150,7 +151,7 @@ def exported_symbols():
     """Names of the C-ABI entry points this binding expects."""
     return [
         "ifosb_create", "ifosb_destroy", "ifosb_last_error", "ifosb_device_bytes", "ifosb_set_cpml",
-        "ifosb_set_model", "ifosb_set_receivers", "ifosb_set_frequencies", "ifosb_forward", "ifosb_residual",
+        "ifosb_set_model", "ifosb_set_model_interior", "ifosb_set_receivers", "ifosb_set_frequencies", "ifosb_forward", "ifosb_residual",
         "ifosb_adjoint", "ifosb_gradient", "ifosb_zero_gradient", "ifosb_get_gradient", "ifosb_shot_gradient",
         "ifosb_get_field", "ifosb_set_launch_mode", "ifosb_last_launch_count", "ifosb_graph_captures", "ifosb_cpml_coeff",
         "ifosb_wavelet", "ifosb_nsamples", "ifosb_moduli", "ifosb_set_profiling", "ifosb_kernel_times",
@@ -289,12 +290,16 @@ class Engine:
         self._c(lib().ifosb_set_cpml(self.h, _p(coeff)))
 
     def set_model(self, rho, pi, u, taus=None, taup=None, eta=None, ghosted=False):
-        """Interior [NY][NX][NZ] arrays (wrapped here like matcopy on one rank) or,
-        with ghosted=True, the caller's own [NY+2][NX+2][NZ+2] arrays."""
-        w = (lambda a: _f32(a)) if ghosted else (lambda a: None if a is None else ghost_wrap(a))
-        arrs = [w(rho), w(pi), w(u), w(taus), w(taup), _f32(eta)]
+        """Interior [NY][NX][NZ] arrays (wrapped on the device like matcopy on one rank)
+        or, with ghosted=True, the caller's own [NY+2][NX+2][NZ+2] arrays."""
+        arrs = [_f32(a) for a in (rho, pi, u, taus, taup, eta)]
+        shape = (self.p.ny, self.p.nx, self.p.nz)
+        inner = not ghosted and all(a is None or a.shape == shape for a in arrs[:5])
+        if not ghosted and not inner:
+            arrs[:5] = [None if a is None else ghost_wrap(a) for a in arrs[:5]]
         self._keep = arrs
-        self._c(lib().ifosb_set_model(self.h, *[_p(a) for a in arrs]))
+        fn = lib().ifosb_set_model_interior if inner else lib().ifosb_set_model
+        self._c(fn(self.h, *[_p(a) for a in arrs]))
 
     def set_surface_moduli(self, pi=None, u=None, ghosted=False):
         """Moduli of the elastic free surface at j = 1 when they differ from the

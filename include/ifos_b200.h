@@ -97,6 +97,11 @@ int ifosb_set_cpml(ifosb_engine *e, const float *coeff);
 int ifosb_set_model(ifosb_engine *e, const float *rho, const float *pi, const float *u,
                     const float *taus, const float *taup, const float *eta);
 
+/* The same from interior arrays [NY][NX][NZ]: the ghost layers, matcopy's periodic
+ * copies on one rank, are made on the device. */
+int ifosb_set_model_interior(ifosb_engine *e, const float *rho, const float *pi, const float *u,
+                             const float *taus, const float *taup, const float *eta);
+
 /* The moduli the elastic free surface uses at j = 1, when they are not the
  * propagation model's: the reference's step-length forwards propagate in the test
  * model but call surface_elastic with the current model's u and pi
