@@ -66,17 +66,24 @@ def slab_memberships(p) -> float:
     return m / n
 
 
-def alg_bytes_per_cell_step(p, nf: int, ntast: int) -> dict:
+DFT_STEPS = 8  # DFT steps the engine takes into the accumulators in one pass, at most
+
+
+def alg_bytes_per_cell_step(p, nf: int, ntast: int, dft_steps: int = 1) -> dict:
     """Compulsory HBM bytes per cell-update: every live state word read and written
     once, every model word read once, averaged moduli counted as recomputable.
-    Split between the two kernels of a step (velocity / stress)."""
+    Split between the two kernels of a step (velocity / stress, which carries the DFT).
+    dft_steps: DFT steps that share a pass over the accumulators; with more than one
+    the pass reads the steps' velocities again."""
     L = p.nmech
     slab = slab_memberships(p)
     vel = 4 * (3 + 3) + 4 * 1 + 24 * slab            # v R+W, rho, 3 psi R+W per slab
     stress = 4 * (6 + 6) + 4 * 2 + 24 * slab          # sigma R+W, pi, u, 3 psi R+W per slab
     if L:
         stress += 48 * L + 8                           # 6 r R+W per mechanism, taus, taup
-    stress += 48.0 * nf / max(ntast, 1)                # 6 DFT accumulators R+W per frequency
+    stress += 48.0 * nf / max(ntast, 1) / dft_steps    # 6 DFT accumulators R+W per frequency
+    if nf and dft_steps > 1:
+        stress += 12.0 / max(ntast, 1)
     return dict(vel=vel, stress=stress, total=vel + stress)
 
 
@@ -492,7 +499,7 @@ def main():
     eng.forward(shots, want_sections=False)
     tv, ts, nsteps = eng.kernel_times()
     eng.set_profiling(False)
-    b = alg_bytes_per_cell_step(p, nf if wl == "elastic128" else 0, c["ntast"])
+    b = alg_bytes_per_cell_step(p, nf if wl == "elastic128" else 0, c["ntast"], DFT_STEPS)
     ncell = p.nx * p.ny * p.nz
     peak, peak_kind = load_peaks()
     ach_step = b["total"] * ncell / ((tv + ts) / nsteps / 1000.0) / 1e9
@@ -678,7 +685,7 @@ def batched_gradient_workload(args, world, rank, local, dist):
     eng.shot_gradient([shots[i] for i in mine[:B]], obs[mine[:B]])
     atv, ats, ansteps = eng.kernel_times()  # the adjoint loop of that shot-gradient
     eng.set_profiling(False)
-    b = alg_bytes_per_cell_step(p, nf, c["ntast"])
+    b = alg_bytes_per_cell_step(p, nf, c["ntast"], DFT_STEPS)
     peak, peak_kind = load_peaks()
     cb = ncell * B
     ach = b["total"] * cb / ((tv + ts) / nsteps / 1000.0) / 1e9
@@ -815,7 +822,7 @@ def visco256_forward(torch, ifosb, synth, dev, stream, steps=2):
     tv, ts, n = e.kernel_times()
     e.close()
     ncell = p.nx * p.ny * p.nz
-    b = alg_bytes_per_cell_step(p, 0, 1)
+    b = alg_bytes_per_cell_step(p, 0, 1, DFT_STEPS)
     peak, _ = load_peaks()
     ach = b["total"] * ncell / ((tv + ts) / n / 1000.0) / 1e9
     return {"workload": "visco256: L=3 forward modelling, 256^3, NT=3000, 400 receivers, 1 shot",

@@ -1,8 +1,9 @@
 // See ifosb_copy.h. The driver's own path for pageable memory is one thread that copies
-// through its staging buffer (12.7 GB/s up, 20 down, 4.6 down into fresh pages on a
-// 16-core host). With these: a 44 MB result into a fresh array 9.6 -> 3 ms, the five
-// fields of a 131x101x150 model 3.3 -> 1.5 ms, a model update at 128^3 (102 MB both ways)
-// 7.2 -> 5.7 ms.
+// through its staging buffer: 12 to 20 GB/s, and 2.3 GB/s into pages nobody has touched.
+// On a 16-core host a 24 MB result arrives in a fresh array in 2.5 ms instead of 11.0 (the
+// threads fault its pages in side by side), a model update at 128^3 (102 MB of arrays that
+// are not in the caches, both ways) takes 5.7 ms instead of 7.2. Below the limits starting
+// the threads costs more than they save (5 MB from a cached array: 0.34 ms against 0.28).
 #include "ifosb_copy.h"
 
 #include <algorithm>
@@ -17,7 +18,7 @@ namespace {
 
 constexpr size_t CHUNK = 1 << 20;       // bytes of a pinned chunk
 constexpr int MAXT = 8, SLOTS = 2;      // threads, chunks each: 16 MB pinned at most
-constexpr size_t LEAST = 4 * CHUNK;     // smaller copies are left to the driver
+constexpr size_t LEAST = 8 * CHUNK, LEAST_RESULT = 4 * CHUNK;  // smaller: the driver's path
 
 struct Pool {
     std::mutex m;  // held through a copy: one at a time uses the chunks, others take the driver's path
@@ -105,17 +106,22 @@ void host_copy_release() {
     if (--pool().refs == 0) pool().free_all();
 }
 
-cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st, bool result) {
     Pool &p = pool();
-    const int parts = host_parts(bytes);
+    // a few MB a thread; less where pages are to be faulted in
+    const int most = host_parts(bytes), parts = result ? most : std::min(most, std::max(2, host_parts(bytes / 3)));
     int dev = 0;
-    const bool up = bytes >= LEAST && parts > 1 && pageable(src), down = bytes >= LEAST && parts > 1 && !up && pageable(dst);
+    const bool up = bytes >= LEAST && parts > 1 && pageable(src);
+    const bool down = !up && bytes >= (result ? LEAST_RESULT : LEAST) && parts > 1 && pageable(dst);
     std::unique_lock<std::mutex> lock(p.m, std::defer_lock);
-    if (!(up != down) || (up && pageable(dst)) || cudaGetDevice(&dev) != cudaSuccess || !lock.try_lock() || !p.ready(dev))
+    if (!(up || down) || (up && pageable(dst)) || (down && pageable(src)) || cudaGetDevice(&dev) != cudaSuccess || !lock.try_lock() || !p.ready(dev))
         return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
     cudaError_t err[MAXT] = {};
     cudaError_t e = cudaEventRecord(p.start, st);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
+    }
     const size_t n = (bytes + CHUNK - 1) / CHUNK;
     run_parts(parts, [&](int t) {
         cudaError_t r = cudaSetDevice(dev);
@@ -152,7 +158,9 @@ cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st)
         e = err[t];
         if (e == cudaSuccess && up) e = cudaStreamWaitEvent(st, p.done[t], 0);
     }
-    return e;
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();  // whatever kept the chunks from being used (another context, say)
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
 }
 
 }  // namespace ifosb

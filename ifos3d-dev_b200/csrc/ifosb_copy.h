@@ -15,8 +15,8 @@ int host_parts(size_t bytes);
 // dst <- src in the order of `st`, like cudaMemcpyAsync with cudaMemcpyDefault. A large
 // copy from or to pageable memory goes through pinned chunks filled or emptied by a few
 // threads, and the call returns when the host side is done (a copy to the host: when it
-// has arrived).
-cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st);
+// has arrived). result: dst is likely an array nobody has touched yet.
+cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st, bool result = false);
 
 // The pinned chunks are shared by the process's engines and optimisers: made by the
 // first large copy, given back when the last of them goes.

@@ -1835,7 +1835,7 @@ extern "C" int ifosb_gradient_td(ifosb_engine *e, int interval, double *kernels)
         if (e->hook_err != cudaSuccess)
             return fail(e, IFOSB_ECUDA, std::string("time-domain copies: ") + cudaGetErrorString(e->hook_err));
         if ((r = check_unstable(e, nshots))) return r;
-        CU(host_copy(kernels, dk, (size_t)4 * n * sizeof(double), e->stream));
+        CU(host_copy(kernels, dk, (size_t)4 * n * sizeof(double), e->stream, true));
         CU(cudaStreamSynchronize(e->stream));
         // the checkpoints stay in the block (the segments only read them): a repeat
         // call for this forward starts from them
@@ -2021,7 +2021,7 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *g
         k64_fold<<<grd3, blk3, 0, e->stream>>>(g, gr, md, raw, L, chain, fold);
         int r;
         if ((r = check_launch(e, "exact VJP gradient"))) return r;
-        CU(host_copy(gmod, fold, (size_t)nq * n * sizeof(double), e->stream));
+        CU(host_copy(gmod, fold, (size_t)nq * n * sizeof(double), e->stream, true));
         CU(cudaStreamSynchronize(e->stream));
         return IFOSB_OK;
     };
@@ -2153,7 +2153,7 @@ extern "C" int ifosb_get_hessian(ifosb_engine *e, float *hess) {
         std::memset(hess, 0, n * sizeof(float));
         return IFOSB_OK;
     }
-    CU(host_copy(hess, e->d_hess, n * sizeof(float), e->stream));
+    CU(host_copy(hess, e->d_hess, n * sizeof(float), e->stream, true));
     CU(cudaStreamSynchronize(e->stream));
     return IFOSB_OK;
 }
@@ -2172,7 +2172,7 @@ extern "C" int ifosb_get_gradient_q(ifosb_engine *e, double *gradq) {
     if (!e || !gradq) return IFOSB_EARG;
     if (!e->d_gradq) return fail(e, IFOSB_ESTATE, "the Q gradient needs a viscoelastic engine (nmech > 0)");
     const size_t n = (size_t)2 * e->p.nx * e->p.ny * e->p.nz;
-    CU(host_copy(gradq, e->d_gradq, n * sizeof(double), e->stream));
+    CU(host_copy(gradq, e->d_gradq, n * sizeof(double), e->stream, true));
     CU(cudaStreamSynchronize(e->stream));
     return IFOSB_OK;
 }
@@ -2181,8 +2181,8 @@ extern "C" int ifosb_get_gradient(ifosb_engine *e, float *grad, double *grad64) 
     if (!e) return IFOSB_EARG;
     const size_t n = (size_t)3 * e->p.nx * e->p.ny * e->p.nz;
     // host or device destinations (unified addressing)
-    if (grad) CU(host_copy(grad, e->d_grad, n * sizeof(float), e->stream));
-    if (grad64) CU(host_copy(grad64, e->d_grad64, n * sizeof(double), e->stream));
+    if (grad) CU(host_copy(grad, e->d_grad, n * sizeof(float), e->stream, true));
+    if (grad64) CU(host_copy(grad64, e->d_grad64, n * sizeof(double), e->stream, true));
     CU(cudaStreamSynchronize(e->stream));
     return IFOSB_OK;
 }
