@@ -279,7 +279,7 @@ def reference_arm(args, world, rank, dist):
     }), flush=True)
 
 
-NT_VISCO384 = 100  # the batched-gradient configuration names no NT; 100 steps keep a step near 23 s
+NT_VISCO384 = 100  # the batched-gradient configuration names no NT; 100 steps keep a step near 16 s
 
 
 def workload_config(wl, world, nt=None):
@@ -291,7 +291,7 @@ def workload_config(wl, world, nt=None):
                 "grid": [384, 256, 384],
                 "grid_axes": "NX x NY x NZ with y the reference's depth axis: 384 x 384 horizontal (x, z), 256 deep",
                 "nt": nt, "nt_choice": "the configuration names no NT; DT=1e-4 s, NT chosen so that a step "
-                                       "(all 32 shot-gradients) takes about 23 s on one B200",
+                                       "(all 32 shot-gradients) takes about 16 s on one B200",
                 "nmech": 3, "nf": 4, "shots": 32, "receivers": 1024,
                 "parallelism": f"shot-sharded x{world}, FP64 gradient all-reduce per step",
                 "l2_flush": "state+DFT about 11 GB per shot > 126 MB L2"}
