@@ -1878,11 +1878,12 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *g
     double *blk = nullptr;
     int *ibuf = nullptr;
     double *damp = nullptr;
-    CU(cudaMalloc(&blk, total * sizeof(double)));
+    size_t nibuf = 0, namp = 0;
+    int rc = dalloc(e, &blk, total);
+    if (rc) return rc;
     double *md = blk, *ck = md + (size_t)N64 * F, *seg = ck + (size_t)nseg * SZ, *lam = seg + (size_t)(K + 1) * SZ;
     double *ld = lam + SZ, *ls = ld + 9 * (size_t)F, *gq = ls + 9 * (size_t)F, *tr = gq + (size_t)N64 * n;
     double *asrc = tr + ntrace;
-    int rc = IFOSB_OK;
     auto run = [&]() -> int {
         CU(cudaMemsetAsync(blk, 0, total * sizeof(double), e->stream));
         const size_t ng = (size_t)(p.nx + 2) * (p.ny + 2) * (p.nz + 2);
@@ -1930,12 +1931,12 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *g
                     for (int t = 0; t < NT; ++t) amps.push_back(e->td_amp[(size_t)pt.row * NT + t]);
                 }
             const int nsrc = (int)cells.size() / 3;
-            if (ibuf) cudaFree(ibuf);
-            if (damp) cudaFree(damp);
-            ibuf = nullptr;
-            damp = nullptr;
-            CU(cudaMalloc(&ibuf, sizeof(int) * (3 * (size_t)ntr + 3 * (size_t)std::max(nsrc, 1))));
-            CU(cudaMalloc(&damp, sizeof(double) * std::max<size_t>(amps.size(), 1)));
+            int r;
+            dfree(e, &ibuf, nibuf);
+            dfree(e, &damp, namp);
+            nibuf = 3 * (size_t)ntr + 3 * (size_t)std::max(nsrc, 1);
+            namp = amps.size();
+            if ((r = dalloc(e, &ibuf, nibuf)) || (r = dalloc(e, &damp, namp))) return r;
             int *drec = ibuf, *dsrc = ibuf + 3 * ntr;
             CU(cudaMemcpyAsync(drec, rec.data(), sizeof(int) * 3 * ntr, cudaMemcpyHostToDevice, e->stream));
             if (nsrc) {
@@ -1961,7 +1962,6 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *g
                     CU(cudaMemcpyAsync(ck + (size_t)(nt / K) * SZ, w, SZ * sizeof(double), cudaMemcpyDeviceToDevice,
                                        e->stream));
             }
-            int r;
             if ((r = check_launch(e, "exact VJP forward"))) return r;
             CU(cudaMemcpyAsync(trh.data(), tr, ntrace * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
             CU(cudaStreamSynchronize(e->stream));
@@ -2027,9 +2027,9 @@ static int vjp_exact_moduli(ifosb_engine *e, int interval, bool chain, double *g
     };
     rc = run();
     cudaStreamSynchronize(e->stream);
-    cudaFree(blk);
-    if (ibuf) cudaFree(ibuf);
-    if (damp) cudaFree(damp);
+    dfree(e, &blk, total);
+    dfree(e, &ibuf, nibuf);
+    dfree(e, &damp, namp);
     return rc;
 }
 

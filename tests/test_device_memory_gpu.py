@@ -1,0 +1,62 @@
+"""Calls that need device memory while an engine holds its velocity ring, which it takes
+from memory that is free and needs for speed alone: the ring makes way, the call works as
+on an empty device, and the engine's later calls give the same bits without it."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from helpers import engine_for
+from ifosb import synth
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+NX, NY, NZ, NT, SHOTS = 64, 56, 60, 24, 40
+PZ = (NZ + 10 + 7) // 8 * 8
+FIELD = (NY + 5) * (NX + 4) * PZ  # floats of a field with its halos
+RING = 7 * 3 * FIELD * 4 * SHOTS
+
+
+@contextlib.contextmanager
+def little_memory(leave):
+    """All of the device's free memory but `leave` bytes taken by somebody else."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    taken = torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del taken
+        torch.cuda.empty_cache()
+
+
+def engine_with_ring(free_surf):
+    """An engine that has run a forward with frequencies and holds the whole ring."""
+    c = synth.small_case(nx=NX, ny=NY, nz=NZ, nt=NT, free_surf=free_surf, nshots=1, ntr=7, seed=4, finv=(300.0,))
+    e, _, _, shots = engine_for(c, max_shots=SHOTS)
+    before = e.device_bytes
+    traces = e.forward(shots)
+    assert e.device_bytes - before >= RING, "no ring to give back"
+    e.residual((traces * np.float32(0.9)).astype(np.float32))
+    return e, shots, traces
+
+
+@pytest.mark.parametrize("free_surf", [0, 1])
+def test_exact_vjp_takes_the_ring(free_surf):
+    e, shots, traces = engine_with_ring(free_surf)
+    dft = e.get_dft(0)
+    want, want_mis = e.vjp_exact(12, moduli=True)
+    held = e.device_bytes
+    # 2 checkpoints, 13 states of a segment and the adjoint's, of 9 fields and their PML
+    # memories in double: more than is free, less than that and the ring
+    with little_memory(16 * 9 * FIELD * 8):
+        got, mis = e.vjp_exact(12, moduli=True)
+    assert e.device_bytes <= held - RING
+    assert np.array_equal(got, want) and np.array_equal(mis, want_mis)
+    assert np.array_equal(e.forward(shots), traces)
+    assert np.array_equal(e.get_dft(0), dft), "DFT fields without the ring"
+    e.close()
