@@ -10,11 +10,13 @@
 #include "ifosb_kernels.cuh"
 #include "ifosb_copy.h"
 #include "ifosb_corr.cuh"
+#include "ifosb_mem.h"
 #include "ifosb_vjp.cuh"
 
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -45,6 +47,33 @@ struct GraphSet {
 
 struct HostPt {
     int s, j, i, k, kind, row;
+};
+
+// Velocity ring: `slots` snapshots of [max_shots][3][field] beside the state's own, so that
+// the DFT takes several steps per pass over its accumulators (attach_ring). `busy` is held
+// while a loop may be using them; at any other time they are given back to whoever finds no
+// device memory: this engine, another one, an optimiser. Graphs captured with the ring name
+// it in their key and are not replayed without it.
+struct Ring : Spare {
+    float *d = nullptr;
+    int slots = 0;
+    int most = MAXRING - 1;
+    size_t one = 0;      // bytes of a slot
+    bool tried = false;  // one look per engine: a batch keeps its launch graphs
+    std::mutex busy;
+    std::atomic<long long> *dev_bytes = nullptr;
+    bool give_back() override {
+        std::unique_lock<std::mutex> l(busy, std::try_to_lock);
+        if (!l.owns_lock()) return false;
+        free_it();
+        return true;
+    }
+    void free_it() {
+        cudaFree(d);
+        *dev_bytes -= (long long)(slots * one);
+        d = nullptr;
+        slots = 0;
+    }
 };
 
 }  // namespace
@@ -86,7 +115,7 @@ struct ifosb_engine {
     bool have_model = false, have_cpml = false, fwd_ok = false, res_ok = false, adj_ok = false;
     int launch_mode = 0;
     long long launches = 0;
-    long long dev_bytes = 0;
+    std::atomic<long long> dev_bytes{0};
     GraphSet gfwd, gadj;
     // kernel timing
     int profile = 0;
@@ -132,11 +161,8 @@ struct ifosb_engine {
     int td_ck_K = 0, td_ck_nshots = 0;
     cudaError_t hook_err = cudaSuccess;
     GraphSet gtd;  // time-domain loops, one graph per batch shape and interval
-    // velocity ring: `ring` snapshots of [max_shots][3][field] beside the state's own, so
-    // that the DFT takes several steps per pass over its accumulators (attach_ring)
-    float *d_ring = nullptr;
-    int ring = 0;
-    bool ring_tried = false;
+    // velocity ring (attach_ring)
+    Ring ring;
     // TMA boxes (default; IFOSB_TMA=0: neighbours from global memory) and their
     // wait-timeout flag; the failure-path test knobs
     int use_tma = 1;
@@ -167,28 +193,10 @@ static int fail(ifosb_engine *e, int code, const std::string &msg) {
                         std::string(#call) + ": " + cudaGetErrorString(_e));                         \
     } while (0)
 
-static void release_graph(GraphSet &gs);
-static void release_ring(ifosb_engine *e) {
-    if (!e->d_ring) return;
-    if (e->stream) cudaStreamSynchronize(e->stream);
-    release_graph(e->gfwd);
-    release_graph(e->gadj);
-    cudaFree(e->d_ring);
-    e->d_ring = nullptr;
-    e->dev_bytes -= (long long)sizeof(float) * e->ring * 3 * e->g.field * e->max_shots;
-    e->ring = 0;
-}
-
 template <class T>
 static int dalloc(ifosb_engine *e, T **ptr, size_t count) {
     if (count == 0) count = 1;
-    cudaError_t r = cudaMalloc((void **)ptr, count * sizeof(T));
-    if (r != cudaSuccess && e->d_ring) {  // the velocity ring is only taken from memory nobody else wants
-        cudaGetLastError();
-        release_ring(e);
-        r = cudaMalloc((void **)ptr, count * sizeof(T));
-    }
-    if (r != cudaSuccess) {
+    if (device_alloc((void **)ptr, count * sizeof(T)) != cudaSuccess) {
         *ptr = nullptr;
         cudaGetLastError();
         return fail(e, IFOSB_ENOMEM, "cudaMalloc of " + std::to_string(count * sizeof(T)) + " bytes failed");
@@ -307,6 +315,7 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
     e->p = *p;
     e->max_shots = max_shots;
     e->max_nf = max_nf;
+    e->ring.dev_bytes = &e->dev_bytes;
     fd_coeffs(p->fdcoeff, &e->b1, &e->b2);
     Geo &g = e->g;
     g.nx = p->nx; g.ny = p->ny; g.nz = p->nz; g.fw = p->fw; g.free_surf = p->free_surf ? 1 : 0; g.nmech = p->nmech;
@@ -331,6 +340,9 @@ extern "C" int ifosb_create(const ifosb_params *p, int max_shots, int max_nf, if
         const int t = atoi(v);
         if (t == 7 || t == 8) e->vby = t;
     }
+    // most slots of the velocity ring (IFOSB_DFT_SLOTS=0..7): for a process that shares the
+    // device with allocators which cannot ask for the ring (torch, another process)
+    if (const char *v = getenv("IFOSB_DFT_SLOTS")) e->ring.most = std::max(0, std::min(atoi(v), MAXRING - 1));
     g.ntk = (p->nz + BX - 1) / BX;
     g.nti = (p->nx + g.by - 1) / g.by;
     {
@@ -399,12 +411,13 @@ extern "C" void ifosb_destroy(ifosb_engine *e) {
     release_graph(e->gfwd);
     release_graph(e->gadj);
     release_graph(e->gtd);
+    spare_remove(&e->ring);
     void *bufs[] = {e->d_state, e->d_psi, e->d_model, e->d_rho_w, e->d_dftf, e->d_dftb, e->d_grad, e->d_grad64,
                     e->d_err, e->d_sec, e->d_diff, e->d_obs, e->d_part, e->d_misfit, e->d_l2, e->d_trig_f,
                     e->d_trig_b, e->d_voff, e->d_soff, e->d_vpts, e->d_spts, e->d_amp, e->d_tma_err, e->d_cpg,
                     e->d_mstage, e->d_green, e->d_gsig, e->d_hess, e->d_sec2, e->d_voff_t, e->d_soff_t,
                     e->d_voff_a, e->d_vpts_t, e->d_spts_t, e->d_vpts_a, e->d_amp_t, e->d_gradq, e->d_smod,
-                    e->d_td_blk, e->d_td_k, e->d_ring, e->d_mraw};
+                    e->d_td_blk, e->d_td_k, e->ring.d, e->d_mraw};
     for (void *b : bufs)
         if (b) cudaFree(b);
     for (cudaEvent_t ev : e->events) cudaEventDestroy(ev);
@@ -451,7 +464,7 @@ extern "C" int ifosb_set_stream(ifosb_engine *e, void *stream) {
 }
 
 extern "C" const char *ifosb_last_error(const ifosb_engine *e) { return e ? e->err.c_str() : "no engine"; }
-extern "C" long long ifosb_device_bytes(const ifosb_engine *e) { return e ? e->dev_bytes : 0; }
+extern "C" long long ifosb_device_bytes(const ifosb_engine *e) { return e ? e->dev_bytes.load() : 0; }
 extern "C" long long ifosb_last_launch_count(const ifosb_engine *e) { return e ? e->launches : 0; }
 extern "C" long long ifosb_graph_captures(const ifosb_engine *e) { return e ? e->captures : 0; }
 
@@ -1010,39 +1023,52 @@ static void plan_loop(ifosb_engine *e, Loop &L, int nshots, bool back) {
 // DFT steps: nt % ntast == 0 (ifos3d.c:788).
 static bool dft_step(const ifosb_engine *e, int nt) { return e->nf > 0 && nt % e->ntast == 0; }
 
+// A loop's hold on the ring, from attach_ring until its kernels have ended.
+struct RingUse {
+    ifosb_engine *e;
+    std::unique_lock<std::mutex> l;
+    bool idle = false;  // the stream has been waited for
+    explicit RingUse(ifosb_engine *eng) : e(eng), l(eng->ring.busy) {}
+    ~RingUse() {
+        if (!idle) cudaStreamSynchronize(e->stream);
+    }
+};
+
 // The velocity ring of a loop that accumulates DFT fields. Called last before the loop,
 // when everything else it needs is allocated: the ring takes at most half of the device
 // memory that is free then, in snapshots of the whole batch, up to MAXRING with the
 // state's own (a 384x256x384, L = 3, nf = 4 shot: 2.49 ms per step with 8), and is
-// given back when any later allocation of the engine fails. The time-domain checkpoints
-// of an armed forward read the state's own velocities after every step: no ring.
+// given back, for good, when any later allocation of the library on this device fails.
+// The time-domain checkpoints of an armed forward read the state's own velocities after
+// every step: no ring.
 static int attach_ring(ifosb_engine *e, Loop &L) {
     L.ring = 1;
     L.slot[0] = e->d_state;
     L.slot_shot[0] = e->st_shot;
     const long long F = e->g.field;
     if (L.dft && e->nf > 0 && L.td.K == 0) {
-        const int want = std::min(MAXRING, e->p.nt / e->ntast) - 1;  // no more snapshots than DFT steps
-        const size_t one = sizeof(float) * 3 * (size_t)F * e->max_shots;
-        if (!e->d_ring && want > 0 && !e->ring_tried) {
+        Ring &r = e->ring;
+        const int want = std::min(r.most, e->p.nt / e->ntast - 1);  // no more snapshots than DFT steps
+        if (!r.d && want > 0 && !r.tried) {
             size_t free_b = 0, total_b = 0;
-            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
-            int n = (int)std::min<size_t>(want, free_b / 2 / one);
-            if (n > 0 && cudaMalloc((void **)&e->d_ring, n * one) != cudaSuccess) n = 0;
-            cudaGetLastError();
-            e->ring_tried = true;  // one look per engine: a batch keeps its launch graphs
-            if (n > 0) {
-                e->ring = n;
-                e->dev_bytes += (long long)(n * one);
-                CU(cudaMemsetAsync(e->d_ring, 0, n * one, e->stream));  // halos stay zero
+            r.one = sizeof(float) * 3 * (size_t)F * e->max_shots;
+            if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || cudaGetDevice(&r.device) != cudaSuccess) free_b = 0;
+            const int n = (int)std::min<size_t>(want, free_b / 2 / r.one);
+            r.tried = true;
+            if (n > 0 && cudaMalloc((void **)&r.d, n * r.one) == cudaSuccess) {
+                r.slots = n;
+                e->dev_bytes += (long long)(n * r.one);
+                spare_add(&r);
+                CU(cudaMemsetAsync(r.d, 0, n * r.one, e->stream));  // halos stay zero
             } else {
-                e->d_ring = nullptr;
+                r.d = nullptr;
             }
+            cudaGetLastError();
         }
-        L.ring = 1 + std::max(0, std::min(want, e->ring));
-        for (int r = 1; r < L.ring; ++r) {
-            L.slot[r] = e->d_ring + (size_t)(r - 1) * 3 * F * e->max_shots;
-            L.slot_shot[r] = 3 * F;
+        L.ring = 1 + std::max(0, std::min(want, r.slots));
+        for (int q = 1; q < L.ring; ++q) {
+            L.slot[q] = r.d + (size_t)(q - 1) * 3 * F * e->max_shots;
+            L.slot_shot[q] = 3 * F;
         }
     }
     // a step after a DFT step whose velocities are still wanted goes to the next slot
@@ -1464,13 +1490,17 @@ extern "C" int ifosb_forward(ifosb_engine *e, int nshots, const ifosb_shot *shot
         L.td = TdHook{uf, uf_end, uf_end + tl.us, tl.ck, tl.ss, tl.ps, tl.us, tl.ssz, tl.psz, tl.K, tl.nseg};
         CU(cudaMemsetAsync(uf, 0, tl.us * sizeof(float), e->stream));
     }
-    if ((rc = finish_plan(e, L))) return rc;
-    e->hook_err = cudaSuccess;
-    if ((rc = run_loop(e, L))) return rc;
-    if (e->hook_err != cudaSuccess)
-        return fail(e, IFOSB_ECUDA, std::string("time-domain checkpoints: ") + cudaGetErrorString(e->hook_err));
-    e->nshots = nshots;
-    if ((rc = check_unstable(e, nshots))) return rc;  // a failed batch is not a forward to build on
+    {
+        RingUse use(e);
+        if ((rc = finish_plan(e, L))) return rc;
+        e->hook_err = cudaSuccess;
+        if ((rc = run_loop(e, L))) return rc;
+        if (e->hook_err != cudaSuccess)
+            return fail(e, IFOSB_ECUDA, std::string("time-domain checkpoints: ") + cudaGetErrorString(e->hook_err));
+        e->nshots = nshots;
+        if ((rc = check_unstable(e, nshots))) return rc;  // a failed batch is not a forward to build on
+        use.idle = true;
+    }
     e->fwd_ok = true;
     if (L.td.K) {
         e->td_ck_ok = true;
@@ -1546,8 +1576,12 @@ extern "C" int ifosb_adjoint(ifosb_engine *e, const float *diff) {
     sa.pts = nullptr;
     L.dft = e->d_dftb;
     L.trig = e->d_trig_b;
-    if ((rc = finish_plan(e, L)) || (rc = run_loop(e, L))) return rc;
-    if ((rc = check_unstable(e, nshots))) return rc;
+    {
+        RingUse use(e);
+        if ((rc = finish_plan(e, L)) || (rc = run_loop(e, L))) return rc;
+        if ((rc = check_unstable(e, nshots))) return rc;
+        use.idle = true;
+    }
     e->adj_ok = true;
     return check_launch(e, "adjoint");
 }
@@ -2100,8 +2134,10 @@ extern "C" int ifosb_hessian_green(ifosb_engine *e, int nrec, const int *rec_ids
         L.sa.pts = nullptr;
         L.dft = dft;
         L.trig = e->d_trig_b;
+        RingUse use(e);
         if ((rc = finish_plan(e, L)) || (rc = run_loop(e, L))) return rc;
         if ((rc = check_unstable(e, B))) return rc;
+        use.idle = true;
     }
     e->ngreen = nrec;
     e->fwd_ok = e->res_ok = e->adj_ok = false;  // the wavefield state now holds the last Green's function

@@ -11,6 +11,7 @@
 // keeps the reference's float/double expressions and is bit-identical to it.
 #include "../../include/ifos_b200.h"
 #include "ifosb_copy.h"
+#include "ifosb_mem.h"
 
 #include <cuda_runtime.h>
 
@@ -352,7 +353,7 @@ extern "C" int ifosb_optim_create(int nx, int ny, int nz, int numpar, int bfgsnu
     o->n = (long long)nx * ny * nz;
     host_copy_retain();
     const long long n = o->n, nn = (long long)numpar * n, mg = (long long)(nx + 2) * (ny + 2) * (nz + 2);
-    auto alloc = [&](void **p, size_t bytes) { return cudaMalloc(p, bytes) == cudaSuccess; };
+    auto alloc = [&](void **p, size_t bytes) { return device_alloc(p, bytes) == cudaSuccess; };
     bool ok = alloc((void **)&o->d_grad, sizeof(float) * 3 * n) && alloc((void **)&o->d_prior, sizeof(float) * 6 * n) &&
               alloc((void **)&o->d_part, sizeof(double) * RBLK * MAXSUM) &&
               alloc((void **)&o->d_sc, sizeof(double) * (2 * bfgsnum + 8)) &&
@@ -595,9 +596,9 @@ extern "C" int ifosb_precon_grad(ifosb_optim *o, float *grad, int damptype, int 
     const size_t ni = src.size() + rec.size();
     float *dt = nullptr;
     int *di = nullptr;
-    OCU(cudaMalloc(&dt, sizeof(float) * nf));
+    OCU(device_alloc((void **)&dt, sizeof(float) * nf));
     if (ni) {
-        cudaError_t ce = cudaMalloc(&di, sizeof(int) * ni);
+        cudaError_t ce = device_alloc((void **)&di, sizeof(int) * ni);
         if (ce != cudaSuccess) {
             cudaFree(dt);
             OCU(ce);
@@ -701,7 +702,7 @@ extern "C" int ifosb_hess_apply(ifosb_optim *o, float *grad, const float *hess, 
     if (!o || !grad || !hess || !water) return IFOSB_EARG;
     const long long n = o->n;
     float *dh = nullptr;
-    OCU(cudaMalloc(&dh, sizeof(float) * 3 * n));
+    OCU(device_alloc((void **)&dh, sizeof(float) * 3 * n));
     cudaError_t ce = host_copy(dh, hess, sizeof(float) * 3 * n, o->stream);
     if (ce == cudaSuccess) ce = host_copy(o->d_grad, grad, sizeof(float) * 3 * n, o->stream);
     if (ce == cudaSuccess) {
@@ -777,8 +778,8 @@ extern "C" int ifosb_resample(const float *src, int nx, int ny, int nz, float dx
     }
     const size_t ns = (size_t)nx * ny * nz, nd = (size_t)mx * my * mz;
     float *ds = nullptr, *dd = nullptr;
-    cudaError_t ce = cudaMalloc(&ds, ns * sizeof(float));
-    if (ce == cudaSuccess) ce = cudaMalloc(&dd, nd * sizeof(float));
+    cudaError_t ce = device_alloc((void **)&ds, ns * sizeof(float));
+    if (ce == cudaSuccess) ce = device_alloc((void **)&dd, nd * sizeof(float));
     if (ce == cudaSuccess) ce = cudaMemcpy(ds, src, ns * sizeof(float), cudaMemcpyDefault);
     if (ce == cudaSuccess) {
         ResampleArgs a{ds, dd, nx, ny, nz, mx, my, mz, (double)ex / (double)dx, (double)ey / (double)dy,

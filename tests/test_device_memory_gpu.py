@@ -6,8 +6,10 @@ import contextlib
 import numpy as np
 import pytest
 
+import ifosb
 from helpers import engine_for
 from ifosb import synth
+from test_gpu_parity import check_case, pick_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -59,4 +61,30 @@ def test_exact_vjp_takes_the_ring(free_surf):
     assert np.array_equal(got, want) and np.array_equal(mis, want_mis)
     assert np.array_equal(e.forward(shots), traces)
     assert np.array_equal(e.get_dft(0), dft), "DFT fields without the ring"
+    e.close()
+
+
+@pytest.mark.parametrize("what", ["engine", "optimiser"])
+def test_other_objects_take_the_ring(what):
+    e, shots, traces = engine_with_ring(1)
+    dft, held = e.get_dft(0), e.device_bytes
+    p = e.p
+    with little_memory(RING // 2):  # more than is free, less than that and the ring
+        if what == "engine":  # the wavefields alone, at 9 fields a shot
+            other = ifosb.Engine(p, max_shots=RING * 3 // 4 // (9 * FIELD * 4), max_nf=0)
+        else:  # two FP64 histories of two parameters
+            other = ifosb.Optimizer(NX, NY, NZ, numpar=2, bfgsnum=RING * 3 // 4 // (2 * 2 * 8 * NX * NY * NZ))
+        assert e.device_bytes == held - RING
+        other.close()
+    assert np.array_equal(e.forward(shots), traces)
+    assert np.array_equal(e.get_dft(0), dft), "DFT fields without the ring"
+    e.close()
+
+
+@pytest.mark.parametrize("slots", [0, 1, 2, 6])
+def test_a_capped_ring_changes_no_bit(slots, oracle, request, monkeypatch):
+    monkeypatch.setenv("IFOSB_DFT_SLOTS", str(slots))
+    c = synth.small_case(nx=19, ny=18, nz=23, nt=25, nshots=2, seed=slots)
+    e, _ = check_case(c, pick_oracle(0, oracle, request))
+    assert e.launch_count == 2 * 25 + -(-25 // (slots + 1)), "passes of slots + 1 DFT steps"
     e.close()
