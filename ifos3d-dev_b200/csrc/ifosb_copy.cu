@@ -160,6 +160,11 @@ cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st,
     }
     if (e == cudaSuccess) return e;
     cudaGetLastError();  // whatever kept the chunks from being used (another context, say)
+    // chunks that are on their way are ordered before nothing on `st`: wait for them
+    for (int t = 0; t < parts; ++t) {
+        e = cudaStreamSynchronize(p.st[t]);
+        if (e != cudaSuccess) return e;
+    }
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
 }
 

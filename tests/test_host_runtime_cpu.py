@@ -4,6 +4,8 @@ callers meet is arranged there, without a GPU."""
 import os
 import subprocess
 
+import pytest
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 FAKE = os.path.join(HERE, "fake_cuda")
 CSRC = os.path.join(os.path.dirname(HERE), "ifos3d-dev_b200", "csrc")
@@ -19,4 +21,17 @@ def build(tmp, check, source):
 def test_memory_that_is_given_back(tmp_path):
     exe = build(tmp_path, "check_mem.cc", "ifosb_mem.cu")
     r = subprocess.run([exe], timeout=60, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+
+
+@pytest.fixture(scope="module")
+def check_copy(tmp_path_factory):
+    return build(tmp_path_factory.mktemp("copy"), "check_copy.cc", "ifosb_copy.cu")
+
+
+@pytest.mark.parametrize("what", ["sizes", "partners", "callers", "failed"])
+def test_host_copies(check_copy, what):
+    """sizes: around a chunk and both limits; partners: pinned and device memory; callers: two
+    at once; failed: a chunk that cannot be sent."""
+    r = subprocess.run([check_copy, what], timeout=120, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
