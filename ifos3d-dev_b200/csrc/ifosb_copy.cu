@@ -123,8 +123,10 @@ cudaError_t host_copy(void *dst, const void *src, size_t bytes, cudaStream_t st,
         return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st);
     }
     const size_t n = (bytes + CHUNK - 1) / CHUNK;
+    const std::thread::id caller = std::this_thread::get_id();
     run_parts(parts, [&](int t) {
-        cudaError_t r = cudaSetDevice(dev);
+        // a new thread has no device yet; the caller's keeps the context it has
+        cudaError_t r = std::this_thread::get_id() == caller ? cudaSuccess : cudaSetDevice(dev);
         if (r == cudaSuccess) r = cudaStreamWaitEvent(p.st[t], p.start, 0);
         auto chunk = [&](size_t c) { return std::min(CHUNK, bytes - c * CHUNK); };
         auto pinned = [&](int s) { return p.pin + ((size_t)t * SLOTS + s) * CHUNK; };

@@ -144,11 +144,23 @@ static int failed() {
     return 0;
 }
 
+// The caller's context stays the calling thread's.
+static int context() {
+    cudaStream_t st = stream();
+    host_copy_retain();
+    fake_context = 5;
+    if (both_ways(20 * MB, st, true, true, true)) return 1;
+    CHECK(fake_context == 5);
+    host_copy_release();
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "sizes") return sizes();
     if (what == "partners") return partners();
     if (what == "callers") return callers();
     if (what == "failed") return failed();
+    if (what == "context") return context();
     return 2;
 }

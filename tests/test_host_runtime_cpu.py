@@ -29,9 +29,9 @@ def check_copy(tmp_path_factory):
     return build(tmp_path_factory.mktemp("copy"), "check_copy.cc", "ifosb_copy.cu")
 
 
-@pytest.mark.parametrize("what", ["sizes", "partners", "callers", "failed"])
+@pytest.mark.parametrize("what", ["sizes", "partners", "callers", "failed", "context"])
 def test_host_copies(check_copy, what):
     """sizes: around a chunk and both limits; partners: pinned and device memory; callers: two
-    at once; failed: a chunk that cannot be sent."""
+    at once; failed: a chunk that cannot be sent; context: the calling thread's stays."""
     r = subprocess.run([check_copy, what], timeout=120, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
