@@ -598,7 +598,6 @@ static int set_model(ifosb_engine *e, const float *rho, const float *pi, const f
         const int rc = dalloc(e, &e->d_mraw, n);
         if (rc) return rc;
     }
-    e->rho_div = rho_range;
     float *tmp = e->d_mstage;
     const float *src[5] = {rho, pi, u, taus, taup};
     for (int q = 0; q < (p.nmech > 0 ? 5 : 3); ++q) {
@@ -621,6 +620,7 @@ static int set_model(ifosb_engine *e, const float *rho, const float *pi, const f
     cudaError_t se = cudaStreamSynchronize(e->stream);
     if (le != cudaSuccess || se != cudaSuccess)
         return fail(e, IFOSB_ECUDA, std::string("av_mat: ") + cudaGetErrorString(le != cudaSuccess ? le : se));
+    e->rho_div = rho_range;
     for (int l = 0; l < MAXMECH; ++l) e->eta[l] = l < p.nmech ? eta[l] : 0.f;
     // readmod() gives every cell the same TAU (readmod.c:57-58, 119-120); then the
     // staggered averages are one value too and the kernels take scalars
