@@ -106,7 +106,10 @@ struct StrBox {
 constexpr int VYB = 2;
 __host__ __device__ constexpr int str_yb(int nmech) { return nmech == 0 ? 2 : 1; }
 
-constexpr unsigned ONE_WAVE = 4 * 148;  // CTAs resident at once
+// CTAs resident at once on a B200 at the four per SM of the launch bounds. (A stress box with
+// four mechanisms and relaxation times per cell is 62 KB: three fit there, and the limits that
+// are counted in waves come a little late.)
+constexpr unsigned ONE_WAVE = 4 * 148;
 
 // This thread's cells in a CTA's box, and the chunk's planes.
 struct BoxAt {

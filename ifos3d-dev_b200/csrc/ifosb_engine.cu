@@ -3,9 +3,9 @@
 // One engine = one device-resident problem: the model (shared by all shots),
 // per-shot wavefield state, PML memory, DFT accumulators and traces for a
 // batch of up to max_shots shots, and the accumulated gradient. The time loops
-// run as two kernels per step (velocity; stress + source + DFT + surface +
-// receivers), captured once into a CUDA graph per batch shape and direction
-// and replayed on later calls.
+// run as two kernels per step (velocity; stress + source + surface + receivers)
+// and a DFT pass over several steps, captured once into a CUDA graph per batch
+// shape and direction and replayed on later calls.
 #include "../../include/ifos_b200.h"
 #include "ifosb_kernels.cuh"
 #include "ifosb_copy.h"
@@ -124,7 +124,7 @@ struct ifosb_engine {
     std::vector<cudaEvent_t> events;
     cudaStream_t own_stream = nullptr;
     // launch shapes picked by ifosb_autotune per batch size: y planes per CTA chunk
-    // and the L2 prefetch distance; nt_limit > 0 shortens the time loop while tuning
+    // and the L2 prefetch distance in boxes; nt_limit > 0 shortens the time loop while tuning
     struct Shape {
         int cyv, l2v, cys, l2s;  // velocity and stress kernels: y planes per chunk, L2 prefetch
     };
@@ -768,7 +768,7 @@ extern "C" int ifosb_set_frequencies(ifosb_engine *e, int nf, const float *finv,
 // ---------------------------------------------------------------------------
 // the time loop
 
-static_assert(TZ == BX && TX == BY, "boxes and the gradient's blocks share the engine's geometry");
+static_assert(TZ == BX, "boxes share the engine's geometry");
 
 // Everything one forward or adjoint call launches with.
 // The time-domain checkpoints an armed forward writes after its steps: the
@@ -2339,7 +2339,7 @@ extern "C" int ifosb_residual_noalloc(int nshots, int ntr, int ns, float dt, con
 
 // Autotuner: for a batch of nshots shots, times `steps` forward time steps
 // (kernel-by-kernel, CUDA events) for each launch shape — y planes per CTA chunk
-// and the L2 prefetch distance of the TMA kernels — and keeps the fastest for
+// and the L2 prefetch distance in boxes of the TMA kernels — and keeps the fastest for
 // later calls with that batch size. The shape changes no arithmetic: results
 // stay bit-identical. The wavefield of the batch is left undefined.
 extern "C" int ifosb_autotune(ifosb_engine *e, int nshots, const ifosb_shot *shots, int steps, int *shape) {
@@ -2351,8 +2351,7 @@ extern "C" int ifosb_autotune(ifosb_engine *e, int nshots, const ifosb_shot *sho
     std::vector<int> cys = {2, 3, 4, 6, 8, 12, 16, 24, 32, 64, hv.cy, hs.cy};
     {
         // chunkings whose CTA count fills one or two waves at 1-4 CTAs per SM: on
-        // a small grid the fixed list leaves either a nearly empty last wave or
-        // chunks so short that each CTA's pipeline start-up dominates
+        // a small grid the fixed list leaves a nearly empty last wave
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         cudaGetLastError();

@@ -15,29 +15,13 @@ __device__ __forceinline__ void mbar_init(uint64_t *b, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *b, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(su32(b)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(b)) : "memory");
-}
-// IFOSB_WAIT_HINT_NS > 0 lets a waiting thread be suspended in hardware for up
-// to that many nanoseconds per try (instead of returning at once and spinning).
-#ifndef IFOSB_WAIT_HINT_NS
-#define IFOSB_WAIT_HINT_NS 0
-#endif
 __device__ __forceinline__ bool mbar_try(uint64_t *b, uint32_t parity) {
     uint32_t ok;
-#if IFOSB_WAIT_HINT_NS > 0
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(su32(b)), "r"(parity), "r"((uint32_t)IFOSB_WAIT_HINT_NS)
-        : "memory");
-#else
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
         : "r"(su32(b)), "r"(parity)
         : "memory");
-#endif
     return ok != 0;
 }
 __device__ __forceinline__ uint64_t gtimer() {

@@ -325,8 +325,8 @@ class Engine:
 
     def set_wait_test(self, wait_ns: int = 1_000_000_000, kernel: int = 0, stop_plane: int = -1):
         """Failure-path test knobs (ifosb_set_wait_test): the TMA kernels' mbarrier
-        wait limit, and the kernel (1 velocity, 2 stress) whose producer warp stops
-        issuing loads at chunk iteration stop_plane. Defaults restore normal runs."""
+        wait limit, and the kernel (1 velocity, 2 stress) whose CTAs issue no loads from
+        box stop_plane of their chunk on. Defaults restore normal runs."""
         self._c(lib().ifosb_set_wait_test(self.h, int(wait_ns), kernel, stop_plane))
 
     def set_launch_mode(self, mode: int):
@@ -381,7 +381,8 @@ class Engine:
 
     def autotune(self, shots, steps=20):
         """Pick the launch shapes for batches of len(shots) shots; returns a dict with
-        the y planes per CTA chunk and L2 prefetch distance of each kernel."""
+        the y planes per CTA chunk and the L2 prefetch distance (in boxes, whatever the
+        key says) of each kernel."""
         arr, keep = self._shots(shots)
         shape = np.zeros(4, np.int32)
         self._c(lib().ifosb_autotune(self.h, len(shots), arr, steps, _p(shape)))

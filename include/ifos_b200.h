@@ -238,14 +238,15 @@ int ifosb_set_launch_mode(ifosb_engine *e, int mode);
  * failures end in err(), src/util.c:30-40). Every mbarrier wait of the TMA time-step
  * kernels gives up after wait_ns (default and maximum 1e9 = 1 s, minimum 1000);
  * the call then returns IFOSB_ECUDA and the engine stays usable. With kernel = 1
- * (velocity) or 2 (stress) and stop_plane >= 0, that kernel's producer warp stops
- * issuing loads at iteration stop_plane of each CTA's y chunk, waits for the boxes
- * it has issued and returns, so the consumers' waits for the rest run out: the
- * path from an expired wait to the error status, made to run without a GPU fault.
+ * (velocity) or 2 (stress) and stop_plane >= 0, that kernel's CTAs issue no loads
+ * from box stop_plane of their y chunk on (a launch shape of several boxes a chunk
+ * has them), so the waits for that box run out: the path from an expired wait to
+ * the error status, made to run without a GPU fault.
  * kernel = 0 (and stop_plane = -1) restores normal launches. For tests only. */
 int ifosb_set_wait_test(ifosb_engine *e, long long wait_ns, int kernel, int stop_plane);
 
-/* Kernels launched by the last forward/adjoint call (per-step kernels x steps). */
+/* Kernels launched by the last forward/adjoint call: two per step, and the DFT passes
+ * (one per 1 to 8 DFT steps, as the velocity ring is long). */
 long long ifosb_last_launch_count(const ifosb_engine *e);
 
 /* Time-loop CUDA graphs captured so far: a call with the same batch shape and
@@ -262,7 +263,7 @@ int ifosb_kernel_times(const ifosb_engine *e, double *vel_ms, double *str_ms, in
 /* Autotuner: times `steps` forward time steps of this batch (the same shots a
  * later ifosb_forward / ifosb_shot_gradient will use) for each launch shape —
  * y planes per CTA chunk (2 to 64, and the built-in choice) and the L2 prefetch
- * distance of the TMA kernels (0-3 planes) — and keeps, for each of the two
+ * distance of the TMA kernels (0-3 boxes of 1 or 2 planes) — and keeps, for each of the two
  * time-step kernels, its fastest shape for every later call with nshots shots.
  * Results do not depend on the shape (bit-identical). The batch's wavefield is
  * undefined afterwards. shape (optional, int[4]) gets the choice: velocity

@@ -68,6 +68,21 @@ __global__ void k_round(const double *x, int n, int *bad, int *first) {
     }
 }
 
+// every float in [2^lo, 2^hi): nrcp4 against the rounded reciprocal
+__global__ void k_reciprocal(int lo, int hi, int *bad, int *first) {
+    const uint32_t q0 = (uint32_t)(lo + 127) << 23, q1 = (uint32_t)(hi + 127) << 23;
+    for (uint32_t q = q0 + 4 * (blockIdx.x * blockDim.x + threadIdx.x); q < q1; q += 4 * gridDim.x * blockDim.x) {
+        F4 b;
+        for (int c = 0; c < 4; ++c) set4(b, c, __uint_as_float(q + c));
+        const F4 r = nrcp4(b);
+        for (int c = 0; c < 4; ++c)
+            if (differ(get4(r, c), -__frcp_rn(get4(b, c)))) {
+                atomicAdd(bad, 1);
+                atomicMin(first, (int)(q + c));
+            }
+    }
+}
+
 int outcome(cudaError_t e, int *d, int *res) {
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(res, d, 2 * sizeof(int), cudaMemcpyDeviceToHost);
@@ -103,6 +118,16 @@ extern "C" int round_check(const double *x, int n, int *res) {
     if (e == cudaSuccess) k_round<<<(n + 127) / 128, 128>>>(d, n, r, r + 1);
     const int rc = outcome(e, r, res);
     cudaFree(d);
+    cudaFree(r);
+    return rc;
+}
+extern "C" int reciprocal_check(int lo, int hi, int *res) {
+    int *r = nullptr;
+    const int init[2] = {0, 0x7fffffff};
+    cudaError_t e = cudaMalloc((void **)&r, sizeof(init));
+    if (e == cudaSuccess) e = cudaMemcpy(r, init, sizeof(init), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) k_reciprocal<<<592, 256>>>(lo, hi, r, r + 1);
+    const int rc = outcome(e, r, res);
     cudaFree(r);
     return rc;
 }

@@ -96,6 +96,13 @@ def test_products_are_not_contracted(check):
     run(check, PRODUCT, with_special(rng, floats(rng, -149, 127)), with_special(rng, floats(rng, -149, 127)), 0)
 
 
+def test_reciprocals(check):
+    """Every divisor of the fast range."""
+    res = (C.c_int * 2)()
+    assert check.reciprocal_check(-10, 24, res) == 0
+    assert res[0] == 0, f"{res[0]} differ, first {np.uint32(res[1]).view(np.float32)!r}"
+
+
 def test_round24(check):
     """A double to float and back, below 2^126: random ones, floats, ties of floats, subnormals."""
     rng = np.random.default_rng(4)

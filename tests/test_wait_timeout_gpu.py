@@ -6,10 +6,9 @@ probe of src/ifos3d.c:761). The engine's counterpart for a TMA stage that never
 lands is a wait limit: each mbarrier wait gives up after the limit, sets an
 error flag, and the call returns IFOSB_ECUDA with the engine still usable.
 
-ifosb_set_wait_test lowers the limit to 1 ms and makes one kernel's producer
-warp stop issuing loads part-way through each y chunk (after the boxes it did
-issue have landed), so the consumers wait on planes that never arrive: a flag
-that nothing sets. The test checks the status, and that the next forward on the
+ifosb_set_wait_test lowers the limit to 1 ms and makes one kernel's CTAs issue no
+loads part-way through each y chunk, so their threads wait on a box that never
+arrives: a flag that nothing sets. The test checks the status, and that the next forward on the
 same engine gives the same bits as before."""
 import numpy as np
 import pytest
@@ -27,7 +26,7 @@ def test_expired_wait_returns_ecuda_and_engine_recovers(nmech, mode):
     c = synth.small_case(nx=40, ny=34, nz=36, nt=30, nmech=nmech, seed=3, nshots=2)
     e, m, cp, shots = engine_for(c)
     e.set_launch_mode(mode)
-    # chunks of 8 planes: a producer that stops at iteration 1 leaves planes unissued
+    # chunks of 8 planes are four boxes or eight: from box 1 on none is issued
     e.set_launch_shape(len(shots), [8, 1, 8, 1])
     ref = e.forward(shots)
     ref_state = e.get_state(1)
