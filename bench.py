@@ -5,7 +5,7 @@
                     [--impl ours|reference]
 
 A step is one pass of the hot path over one batch of synthetic input:
-  visco256   (default) one viscoelastic (L=3) forward modelling run of a shot,
+  visco256   one viscoelastic (L=3) forward modelling run of a shot,
              256^3 cells, NT=3000, 400 receivers — the plain viscoelastic
              forward-modelling configuration; per GPU one shot (shots shard
              across ranks, no data-path collective: weak scaling).
@@ -15,9 +15,9 @@ A step is one pass of the hot path over one batch of synthetic input:
              shot gradients, precon_grad, CG, step-length test forwards, model
              update) on 96x64x96 cells at 2 m, then on 192x128x192 at 1 m
              from the resampled model, 16 shots, three frequency stages.
-  visco384   the batched multi-shot gradient: 32 viscoelastic (L=3) shot-gradients
+  visco384   (default) the batched multi-shot gradient: 32 viscoelastic (L=3) shot-gradients
              (4 frequencies, 1024 receivers) on 384 x 256 x 384 cells, in
-             HBM-sized batches of shots that share one launch; NT=200 by default
+             HBM-sized batches of shots that share one launch; NT=100 by default
              (the configuration names no NT). Shots shard across ranks; one FP64
              all-reduce of gradient and misfits per step.
 metric: cell-updates per second over all ranks (all NX*NY*NZ cells of every
@@ -66,7 +66,12 @@ def slab_memberships(p) -> float:
     return m / n
 
 
-DFT_STEPS = 8  # DFT steps the engine takes into the accumulators in one pass, at most
+def dft_steps_per_pass(eng, p, nf: int, ntast: int) -> float:
+    """DFT steps that shared a pass over the accumulators in the engine's last time loop:
+    up to 8, fewer where its velocity ring found less memory. Two kernels a step, the
+    rest are passes."""
+    passes = eng.launch_count - 2 * p.nt
+    return (p.nt // ntast) / passes if nf and passes > 0 else 1.0
 
 
 def alg_bytes_per_cell_step(p, nf: int, ntast: int, dft_steps: int = 1) -> dict:
@@ -447,14 +452,14 @@ def main():
         t = torch.tensor([ms], device=dev)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms = float(t.item())
-    # our kernels per step: 2 per time step (velocity, stress); a shot-gradient adds the
-    # adjoint loop, residual + misfit and the gradient kernel
-    launches = args.steps * (2 * p.nt if wl == "visco256" else 4 * p.nt + 3)
+    # our kernels per step: a time loop's are 2 per time step (velocity, stress) and its DFT
+    # passes; a shot-gradient has two loops, residual + misfit and the gradient kernel
+    launches = args.steps * (eng.launch_count if wl == "visco256" else 2 * eng.launch_count + 3)
     if td_k:
-        # forward 2 NT + NT sums; residual 2; recomputed steps 2 last + last sums, adjoint
-        # 2 NT + NT sums, last correlations, one dc kernel (last = TIME/DT - 1)
+        # the forward's loop; residual 2; recomputed steps 2 last, adjoint 2 NT, last
+        # correlations, one dc kernel (last = TIME/DT - 1)
         last = round(float(p.time) / float(p.dt)) - 1
-        launches = args.steps * (3 * p.nt + 2 + 3 * last + 3 * p.nt + last + 1)
+        launches = args.steps * (eng.launch_count + 2 + 2 * last + 2 * p.nt + last + 1)
     value = world * cells_step * args.steps / (ms / 1000.0) / 1e9
 
     # ---- end to end through the public API: host model + wavelet in, traces out, every step
@@ -499,7 +504,8 @@ def main():
     eng.forward(shots, want_sections=False)
     tv, ts, nsteps = eng.kernel_times()
     eng.set_profiling(False)
-    b = alg_bytes_per_cell_step(p, nf if wl == "elastic128" else 0, c["ntast"], DFT_STEPS)
+    per_pass = dft_steps_per_pass(eng, p, nf if wl == "elastic128" else 0, c["ntast"])
+    b = alg_bytes_per_cell_step(p, nf if wl == "elastic128" else 0, c["ntast"], per_pass)
     ncell = p.nx * p.ny * p.nz
     peak, peak_kind = load_peaks()
     ach_step = b["total"] * ncell / ((tv + ts) / nsteps / 1000.0) / 1e9
@@ -514,6 +520,7 @@ def main():
                 "traffic": traffic["time_step"] if traffic else None,
                 "traffic_source": traffic["source"] if traffic else "no ncu capture of this workload",
                 "alg_bytes_per_step": round(b["total"] * ncell), "alg_bytes_per_cell_step": round(b["total"], 2),
+                "dft_steps_per_pass": round(per_pass, 2),
                 "per_kernel": {"k_stress": {"alg_bytes_per_cell": round(b["stress"], 2), "ms": round(ts / nsteps, 4),
                                             "achieved_gbs": round(ach_str, 1), "frac": round(ach_str / peak, 4),
                                             "traffic": traffic["k_stress"] if traffic else None},
@@ -651,7 +658,9 @@ def batched_gradient_workload(args, world, rank, local, dist):
     ncell = p.nx * p.ny * p.nz
     cells_step = 2 * ncell * p.nt * nshots
     value = cells_step * args.steps / (ms / 1000.0) / 1e9
-    launches = args.steps * nbatch * (4 * p.nt + 3)
+    # per batch: two time loops (two kernels per time step and the DFT passes), residual +
+    # misfit and the gradient kernel
+    launches = args.steps * nbatch * (2 * eng.launch_count + 3)
 
     # ---- end to end: host model and host observed traces in, FP64 gradient out, every step
     hm = {k: _pinned(torch, ifosb.ghost_wrap(m[k])) for k in ("rho", "pi", "u", "taus", "taup")}
@@ -685,7 +694,8 @@ def batched_gradient_workload(args, world, rank, local, dist):
     eng.shot_gradient([shots[i] for i in mine[:B]], obs[mine[:B]])
     atv, ats, ansteps = eng.kernel_times()  # the adjoint loop of that shot-gradient
     eng.set_profiling(False)
-    b = alg_bytes_per_cell_step(p, nf, c["ntast"], DFT_STEPS)
+    per_pass = dft_steps_per_pass(eng, p, nf, c["ntast"])
+    b = alg_bytes_per_cell_step(p, nf, c["ntast"], per_pass)
     peak, peak_kind = load_peaks()
     cb = ncell * B
     ach = b["total"] * cb / ((tv + ts) / nsteps / 1000.0) / 1e9
@@ -698,6 +708,7 @@ def batched_gradient_workload(args, world, rank, local, dist):
                 "traffic": traffic["time_step"] if traffic else None,
                 "traffic_source": traffic["source"] if traffic else "no ncu capture of this workload",
                 "alg_bytes_per_cell_step": round(b["total"], 2), "alg_bytes_per_step": round(b["total"] * cb),
+                "dft_steps_per_pass": round(per_pass, 2),
                 "per_kernel": {"k_stress": {"alg_bytes_per_cell": round(b["stress"], 2), "ms": round(ts / nsteps, 4),
                                             "achieved_gbs": round(ach_s, 1), "frac": round(ach_s / peak, 4),
                                             "traffic": traffic["k_stress"] if traffic else None},
@@ -822,7 +833,7 @@ def visco256_forward(torch, ifosb, synth, dev, stream, steps=2):
     tv, ts, n = e.kernel_times()
     e.close()
     ncell = p.nx * p.ny * p.nz
-    b = alg_bytes_per_cell_step(p, 0, 1, DFT_STEPS)
+    b = alg_bytes_per_cell_step(p, 0, 1)
     peak, _ = load_peaks()
     ach = b["total"] * ncell / ((tv + ts) / n / 1000.0) / 1e9
     return {"workload": "visco256: L=3 forward modelling, 256^3, NT=3000, 400 receivers, 1 shot",
