@@ -18,7 +18,7 @@
 
 namespace ifosb {
 
-// planes of a CTA: 1 (85 KB, two CTAs per SM at 244 registers) 6.8 ms for 384x256x384, L = 3,
+// planes of a CTA: 1 (85 KB, two CTAs per SM at up to 238 registers) 6.8 ms for 384x256x384, L = 3,
 // nf = 4; 2 planes (106 KB, 128 registers with spills) 8.3, one CTA of 2 planes 7.4
 constexpr int CYB = 1;
 constexpr int CTHR = 16 * 8 * CYB;     // threads: 16 pairs of cells along z

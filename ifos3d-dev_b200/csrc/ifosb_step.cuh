@@ -59,7 +59,7 @@ __device__ __forceinline__ long long szq(const Geo &g, int j, int i, int k) {
 // The quad's place in the CPML frame. Its PML memories are asked for before the update
 // (prefetch into L1, no registers) and read when their axis is done: held in registers
 // from the start, up to nine words a thread, they cost the velocity kernel a fifth of
-// its time at 256^3 (128 registers with spills against 120 without).
+// its time at 256^3 (128 registers with spills against 115 without).
 struct Psi {
     int hx, hy, zm;
     float *px, *py, *pz;
